@@ -39,6 +39,20 @@ def test_matmul_reference(dev, orc, m, n, k):
                 assert orc.close(A @ B + beta * c0[0], got[0], 1e-4)
 
 
+# around the small-tile kernel's rows (4 a thread, 32 a tile), columns and k slices (64, six in a ring), and around the line to the large tiles
+@pytest.mark.parametrize("batch,m,n,k", [(1, 1, 32, 64), (1, 1, 33, 65), (2, 2, 31, 63), (1, 5, 64, 384), (1, 4, 97, 449), (3, 32, 1, 7), (1, 33, 40, 320), (1, 31, 6000, 30),
+                                         (1, 33, 5888, 33), (1, 33, 5889, 33)])
+def test_small_products(dev, orc, batch, m, n, k):
+    for ta in (False, True):
+        for tb in (False, True):
+            a = orc.normal((batch, k, m) if ta else (batch, m, k), 11 + m)
+            b = orc.normal((batch, n, k) if tb else (batch, k, n), 12 + n)
+            c0 = orc.normal((batch, m, n), 13 + k)
+            got = _mm(dev, a, b, c0, batch, m, n, k, ta, tb, 0.5)
+            exp = orc.matmul_f32(a, b, batch, m, n, k, ta, tb, 0.5, c=c0)
+            assert np.array_equal(got.view(np.uint32), exp.reshape(got.shape).view(np.uint32)), (ta, tb)
+
+
 def test_large_tensors(dev, orc):
     a = orc.normal((1000, 1000), 9)
     ones = np.ones((1000, 1), np.float32)

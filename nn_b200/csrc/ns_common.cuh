@@ -142,6 +142,17 @@ NS_DEVINL const T* ns_after_wait(const T* ptr)
 // Lets the next kernel on the stream start its prologue.
 NS_DEVINL void ns_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// True in one lane of a converged warp.  The warps that issue TMA loads and tcgen05 instructions run their loops with all lanes
+// and let the elected one issue: in a loop that a single lane runs (`if (lane == 0)`, divergent control flow) addresses and
+// descriptors stay in per-lane registers and each tcgen05.mma took about 55 cycles to issue, a TMA load about 150 -- 500
+// cycles per k-block, whatever the tile's width (bf16 2048 x 5632, one CTA per 128 columns: 88 k-blocks 28.0 us against 16.4).
+NS_DEVINL bool ns_elect()
+{
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+    return ok != 0;
+}
+
 NS_DEVINL uint32_t ns_smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
 NS_DEVINL void ns_mbar_init(uint32_t bar, uint32_t count)
@@ -201,6 +212,12 @@ NS_DEVINL bool ns_mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_f
         }
     }
     return true;
+}
+
+// The same by all lanes of a converged warp: one verdict for all of them.
+NS_DEVINL bool ns_mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code)
+{
+    return __all_sync(0xffffffffu, ns_mbar_wait(bar, parity, abort_flag, status, code));
 }
 
 // TMA tiled loads, global -> this CTA's shared memory, completion counted on an mbarrier.

@@ -8,9 +8,9 @@
 // (add_rowvec_f32, bias_gelu_f32, add_f32) folded into the epilogue.
 //
 // Shape of one CTA (192 threads, persistent over output tiles):
-//   warp 0      producer: one lane issues the TMA loads of a [128 x 128 B] tile of A and a
-//               [BN x 128 B] tile of B per k-block into a STAGES-deep ring (128-byte swizzle)
-//   warp 1      one lane issues tcgen05.mma (4 per k-block, each 32 bytes of K) into one of two
+//   warp 0      producer: all lanes run its loop, an elected one issues the TMA loads of a [128 x 128 B] tile of A
+//               and a [BN x 128 B] tile of B per k-block into a STAGES-deep ring (128-byte swizzle)
+//   warp 1      likewise, the elected lane issues tcgen05.mma (4 per k-block, each 32 bytes of K) into one of two
 //               accumulators in tensor memory; tcgen05.commit releases the ring slot / hands the
 //               accumulator to the epilogue
 //   warps 2..5  epilogue: each warp owns the 32 accumulator lanes of its quadrant (warp % 4), reads
@@ -340,86 +340,89 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tmA, const CUten
 
     if (warp == 0) {
         // ---------------------------------------------------------------- producer
-        if (lane == 0) {
-            const uint32_t stage_tx = (uint32_t)p.a_rows * BKB + Cfg::B_BYTES;
-            auto load_b = [&](int s, int kb, int tn) {
-                const uint32_t b_dst = smem_base + s * Cfg::STAGE_BYTES + Cfg::A_BYTES;
-                if (!B_MN) {
-                    ns_tma_load_2d(b_dst, &tmB, full_bar(s), kb * ELEMS_PER_KB, tn * BN);
-                } else {
-                    // B stored [K, N]: boxes of 64 columns x 64 rows of K, one per 64 columns of the tile
+        const bool leader = ns_elect();
+        const uint32_t stage_tx = (uint32_t)p.a_rows * BKB + Cfg::B_BYTES;
+        auto load_b = [&](int s, int kb, int tn) {
+            const uint32_t b_dst = smem_base + s * Cfg::STAGE_BYTES + Cfg::A_BYTES;
+            if (!B_MN) {
+                ns_tma_load_2d(b_dst, &tmB, full_bar(s), kb * ELEMS_PER_KB, tn * BN);
+            } else {
+                // B stored [K, N]: boxes of 64 columns x 64 rows of K, one per 64 columns of the tile
 #pragma unroll
-                    for (int c = 0; c < BN / 64; c++)
-                        ns_tma_load_2d(b_dst + c * (64 * 128), &tmB, full_bar(s), tn * BN + c * 64, kb * 64);
-                }
-            };
-            // When B holds weights, which no kernel of the step writes (p.prefetch_b, set by the Linear objects only):
-            // the first ring-full of B tiles is requested before waiting for the previous kernel, so its HBM latency
-            // overlaps that kernel's tail.  A caller's own B may have been written by the kernel just before this one.
-            int armed = 0;
-            if (p.prefetch_b && (int)blockIdx.x < n_items) {
-                int tm, tn, split;
-                tile_coords(p, blockIdx.x, tm, tn, split);
-                const int kb0 = split * p.kb_per_split;
-                const int kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
-                armed = min(STAGES, kb1 - kb0);
-                for (int i = 0; i < armed; i++) {
-                    ns_mbar_expect_tx(full_bar(i), stage_tx);
-                    load_b(i, kb0 + i, tn);
-                }
+                for (int c = 0; c < BN / 64; c++)
+                    ns_tma_load_2d(b_dst + c * (64 * 128), &tmB, full_bar(s), tn * BN + c * 64, kb * 64);
             }
-            ns_pdl_wait();
-            ns_pdl_trigger();
-            int s = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                int tm, tn, split;
-                tile_coords(p, item, tm, tn, split);
-                int kb0 = split * p.kb_per_split;
-                int kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
-                for (int kb = kb0; kb < kb1; kb++) {
-                    const uint32_t a_dst = smem_base + s * Cfg::STAGE_BYTES;
-                    if (armed > 0) {
-                        armed--;   // slot already armed and its B tile on the way
-                    } else {
-                        ok = ns_mbar_wait(empty_bar(s), phase ^ 1u, abort_flag, p.status, p.status_base + 1);
-                        if (!ok) break;
+        };
+        // When B holds weights, which no kernel of the step writes (p.prefetch_b, set by the Linear objects only):
+        // the first ring-full of B tiles is requested before waiting for the previous kernel, so its HBM latency
+        // overlaps that kernel's tail.  A caller's own B may have been written by the kernel just before this one.
+        int armed = 0;
+        if (p.prefetch_b && (int)blockIdx.x < n_items) {
+            int tm, tn, split;
+            tile_coords(p, blockIdx.x, tm, tn, split);
+            const int kb0 = split * p.kb_per_split;
+            const int kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
+            armed = min(STAGES, kb1 - kb0);
+            for (int i = 0; leader && i < armed; i++) {
+                ns_mbar_expect_tx(full_bar(i), stage_tx);
+                load_b(i, kb0 + i, tn);
+            }
+        }
+        ns_pdl_wait();
+        ns_pdl_trigger();
+        int s = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+            int tm, tn, split;
+            tile_coords(p, item, tm, tn, split);
+            int kb0 = split * p.kb_per_split;
+            int kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
+            for (int kb = kb0; kb < kb1; kb++) {
+                const uint32_t a_dst = smem_base + s * Cfg::STAGE_BYTES;
+                if (armed > 0) {
+                    armed--;   // slot already armed and its B tile on the way
+                } else {
+                    ok = ns_mbar_wait_warp(empty_bar(s), phase ^ 1u, abort_flag, p.status, p.status_base + 1);
+                    if (!ok) break;
+                    if (leader) {
                         ns_mbar_expect_tx(full_bar(s), stage_tx);
                         load_b(s, kb, tn);
                     }
-                    ns_tma_load_2d(a_dst, &tmA, full_bar(s), kb * ELEMS_PER_KB, tm * BM);
-                    if (++s == STAGES) { s = 0; phase ^= 1u; }
                 }
+                if (leader) ns_tma_load_2d(a_dst, &tmA, full_bar(s), kb * ELEMS_PER_KB, tm * BM);
+                if (++s == STAGES) { s = 0; phase ^= 1u; }
             }
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc = KIND == NS_KIND_I8 ? ns_idesc(2, 1, 0, 0, BM, BN) : ns_idesc(1, 1, 0, B_MN ? 1 : 0, BM, BN);
-            const uint64_t desc_k = ns_desc_base(16, 1024);            // K-major: 8-row groups 1024 B apart
-            const uint64_t desc_mn = ns_desc_base(64 * 128, 1024);     // MN-major: 64-column blocks 8 KB apart, 8 k-rows 1 KB apart
-            int s = 0;
-            uint32_t phase = 0;
-            int local = 0;
-            bool ok = true;
-            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, local++) {
-                int tm, tn, split;
-                tile_coords(p, item, tm, tn, split);
-                int kb0 = split * p.kb_per_split;
-                int kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
-                const int acc = local & 1;
-                const uint32_t acc_phase = (local >> 1) & 1;
-                ok = ns_mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, p.status, p.status_base + 2);
+        const bool leader = ns_elect();
+        const uint32_t tmem_all = __shfl_sync(0xffffffffu, tmem_base, 0);
+        constexpr uint32_t idesc = KIND == NS_KIND_I8 ? ns_idesc(2, 1, 0, 0, BM, BN) : ns_idesc(1, 1, 0, B_MN ? 1 : 0, BM, BN);
+        const uint64_t desc_k = ns_desc_base(16, 1024);            // K-major: 8-row groups 1024 B apart
+        const uint64_t desc_mn = ns_desc_base(64 * 128, 1024);     // MN-major: 64-column blocks 8 KB apart, 8 k-rows 1 KB apart
+        int s = 0;
+        uint32_t phase = 0;
+        int local = 0;
+        bool ok = true;
+        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, local++) {
+            int tm, tn, split;
+            tile_coords(p, item, tm, tn, split);
+            int kb0 = split * p.kb_per_split;
+            int kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
+            const int acc = local & 1;
+            const uint32_t acc_phase = (local >> 1) & 1;
+            ok = ns_mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, abort_flag, p.status, p.status_base + 2);
+            if (!ok) break;
+            ns_tc_fence_after();
+            const uint32_t d_tmem = tmem_all + acc * BN;
+            for (int kb = kb0; kb < kb1; kb++) {
+                ok = ns_mbar_wait_warp(full_bar(s), phase, abort_flag, p.status, p.status_base + 3);
                 if (!ok) break;
                 ns_tc_fence_after();
-                const uint32_t d_tmem = tmem_base + acc * BN;
-                for (int kb = kb0; kb < kb1; kb++) {
-                    ok = ns_mbar_wait(full_bar(s), phase, abort_flag, p.status, p.status_base + 3);
-                    if (!ok) break;
-                    ns_tc_fence_after();
-                    const uint32_t a_addr = smem_base + s * Cfg::STAGE_BYTES;
-                    const uint32_t b_addr = a_addr + Cfg::A_BYTES;
+                const uint32_t a_addr = smem_base + s * Cfg::STAGE_BYTES;
+                const uint32_t b_addr = a_addr + Cfg::A_BYTES;
+                if (leader) {
 #pragma unroll
                     for (int kk = 0; kk < 4; kk++) {
                         const uint64_t a_desc = ns_desc_at(desc_k, a_addr + kk * 32);
@@ -429,10 +432,10 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tmA, const CUten
                         else ns_mma_f16(d_tmem, a_desc, b_desc, idesc, accumulate);
                     }
                     ns_tc_commit(empty_bar(s));
-                    if (++s == STAGES) { s = 0; phase ^= 1u; }
                 }
-                if (ok) ns_tc_commit(tfull_bar(acc));
+                if (++s == STAGES) { s = 0; phase ^= 1u; }
             }
+            if (ok && leader) ns_tc_commit(tfull_bar(acc));
         }
     } else if (warp < 6) {
         // ---------------------------------------------------------------- epilogue
@@ -703,19 +706,20 @@ ns_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
     if (warp == 0) {
         // ---------------------------------------------------------------- producer (both CTAs)
-        if (lane == 0) {
-            int s = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            for (int i = 0; i < work.count && ok; i++) {
-                int item, kb0, kb1, role, tm, tn;
-                pair_item(p, work, cluster, n_clusters, i, item, kb0, kb1, role);
-                pair_coords(p, item, tm, tn);
-                const int row0 = tm * 256 + (int)rank * BM;
-                const int brow0 = tn * BN + (int)rank * Cfg::BN_HALF;
-                for (int kb = kb0; kb < kb1; kb++) {
-                    ok = ns_mbar_wait(empty_bar(s), phase ^ 1u, abort_flag, p.status, p.status_base + 11);
-                    if (!ok) break;
+        const bool leader = ns_elect();
+        int s = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int i = 0; i < work.count && ok; i++) {
+            int item, kb0, kb1, role, tm, tn;
+            pair_item(p, work, cluster, n_clusters, i, item, kb0, kb1, role);
+            pair_coords(p, item, tm, tn);
+            const int row0 = tm * 256 + (int)rank * BM;
+            const int brow0 = tn * BN + (int)rank * Cfg::BN_HALF;
+            for (int kb = kb0; kb < kb1; kb++) {
+                ok = ns_mbar_wait_warp(empty_bar(s), phase ^ 1u, abort_flag, p.status, p.status_base + 11);
+                if (!ok) break;
+                if (leader) {
                     // the even CTA's barrier counts the four boxes of the pair (boxes that reach past the matrix
                     // edge are zero-filled and still count in full)
                     if (rank == 0) ns_mbar_expect_tx(full_bar(s), 2 * Cfg::STAGE_BYTES);
@@ -729,18 +733,20 @@ ns_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                         ns_tma_load_2d_pair(a_dst + Cfg::A_BYTES, &tmB, bar, brow0, kb * 64);
                         ns_tma_load_2d_pair(a_dst + Cfg::A_BYTES + 64 * 128, &tmB, bar, brow0 + 64, kb * 64);
                     }
-                    if (++s == STAGES) { s = 0; phase ^= 1u; }
                 }
-            }
-            // the commits that free the last ring slots arrive in this CTA's shared memory: see them land before leaving
-            for (int i = 0; i < STAGES && ok; i++) {
-                ok = ns_mbar_wait(empty_bar(s), phase ^ 1u, abort_flag, p.status, p.status_base + 15);
                 if (++s == STAGES) { s = 0; phase ^= 1u; }
             }
         }
+        // the commits that free the last ring slots arrive in this CTA's shared memory: see them land before leaving
+        for (int i = 0; i < STAGES && ok; i++) {
+            ok = ns_mbar_wait_warp(empty_bar(s), phase ^ 1u, abort_flag, p.status, p.status_base + 15);
+            if (++s == STAGES) { s = 0; phase ^= 1u; }
+        }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer (even CTA only)
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
+            const bool leader = ns_elect();
+            const uint32_t tmem_all = __shfl_sync(0xffffffffu, tmem_base, 0);
             constexpr uint32_t idesc = KIND == NS_KIND_I8 ? ns_idesc(2, 1, 0, 0, 256, BN) : ns_idesc(1, 1, 0, B_MN ? 1 : 0, 256, BN);
             const uint64_t desc_k = ns_desc_base(16, 1024);
             const uint64_t desc_mn = ns_desc_base(64 * 128, 1024);     // MN-major: 64-column blocks 8 KB apart, 8 k-rows 1 KB apart
@@ -753,28 +759,30 @@ ns_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 pair_item(p, work, cluster, n_clusters, i, item, kb0, kb1, role);
                 const int acc = local & 1;
                 const uint32_t acc_phase = (local >> 1) & 1;
-                ok = ns_mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, p.status, p.status_base + 12);
+                ok = ns_mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, abort_flag, p.status, p.status_base + 12);
                 if (!ok) break;
                 ns_tc_fence_after();
-                const uint32_t d_tmem = tmem_base + acc * BN;
+                const uint32_t d_tmem = tmem_all + acc * BN;
                 for (int kb = kb0; kb < kb1; kb++) {
-                    ok = ns_mbar_wait(full_bar(s), phase, abort_flag, p.status, p.status_base + 13);
+                    ok = ns_mbar_wait_warp(full_bar(s), phase, abort_flag, p.status, p.status_base + 13);
                     if (!ok) break;
                     ns_tc_fence_after();
                     const uint32_t a_addr = smem_base + s * Cfg::STAGE_BYTES;
                     const uint32_t b_addr = a_addr + Cfg::A_BYTES;
+                    if (leader) {
 #pragma unroll
-                    for (int kk = 0; kk < 4; kk++) {
-                        const uint64_t a_desc = ns_desc_at(desc_k, a_addr + kk * 32);
-                        const uint64_t b_desc = B_MN ? ns_desc_at(desc_mn, b_addr + kk * (16 * 128)) : ns_desc_at(desc_k, b_addr + kk * 32);
-                        const uint32_t accumulate = (kb > kb0 || kk > 0) ? 1u : 0u;
-                        if (KIND == NS_KIND_I8) ns_mma_i8_pair(d_tmem, a_desc, b_desc, idesc, accumulate);
-                        else ns_mma_f16_pair(d_tmem, a_desc, b_desc, idesc, accumulate);
+                        for (int kk = 0; kk < 4; kk++) {
+                            const uint64_t a_desc = ns_desc_at(desc_k, a_addr + kk * 32);
+                            const uint64_t b_desc = B_MN ? ns_desc_at(desc_mn, b_addr + kk * (16 * 128)) : ns_desc_at(desc_k, b_addr + kk * 32);
+                            const uint32_t accumulate = (kb > kb0 || kk > 0) ? 1u : 0u;
+                            if (KIND == NS_KIND_I8) ns_mma_i8_pair(d_tmem, a_desc, b_desc, idesc, accumulate);
+                            else ns_mma_f16_pair(d_tmem, a_desc, b_desc, idesc, accumulate);
+                        }
+                        ns_tc_commit_pair(empty_bar(s), 3);       // the ring slot is free in both CTAs
                     }
-                    ns_tc_commit_pair(empty_bar(s), 3);       // the ring slot is free in both CTAs
                     if (++s == STAGES) { s = 0; phase ^= 1u; }
                 }
-                if (ok) ns_tc_commit_pair(tfull_bar(acc), 3);   // both CTAs' epilogues may read their accumulator
+                if (ok && leader) ns_tc_commit_pair(tfull_bar(acc), 3);   // both CTAs' epilogues may read their accumulator
             }
         }
     } else {

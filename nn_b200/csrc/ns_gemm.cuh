@@ -12,7 +12,7 @@ struct NsGemmParams {
     int k_splits;       // >= 1
     int kb_per_split;   // k-blocks per split
     int tiles_m, tiles_n;
-    int a_rows;         // rows of A fetched per tile (64 when M <= 64, else 128)
+    int a_rows;         // rows of A fetched per tile (M in whole groups of 8, at most 128)
     int epilogue;       // NS_EPI_*
     int out_dtype;      // NS_F32 / NS_BF16
     int residual_dtype;

@@ -1043,11 +1043,6 @@ void ns_gemm_choose_tiling(const NsDevice* d, int M, int N, int k_blocks, int* b
     } else if (tiles_m == 1) {
         bn = b_is_kn ? 256 : 128;
         while (bn > 64 && bn / 2 >= N) bn >>= 1;
-        // 64-wide tiles that fill one wave by themselves need no split and no second kernel.  A k-block of such a tile costs almost
-        // what one of 128 columns costs, so only while there are few: N = 8192, 32 k-blocks, 64 rows 9.9 against 12.6 us (bf16); with
-        // 64 k-blocks (N = 8192, K = 4096) the two are level.
-        const int narrow = (N + 63) / 64;
-        if (!b_is_kn && k_blocks <= 32 && narrow <= d->sm_count && narrow * 2 > d->sm_count) bn = 64;
     } else {
         while (bn > 64 && tiles_m * ((N + bn - 1) / bn) < d->sm_count) bn >>= 1;
         while (bn > 64 && bn / 2 >= N) bn >>= 1;

@@ -134,9 +134,8 @@ def test_cta_pair_kernel_with_k_blocks_dealt_out_evenly(dev, orc, m, n, k, trans
     assert np.array_equal(c1.view(np.uint32), c2.view(np.uint32))
 
 
-# fetched rows come in groups of 8 (1 .. 128); 64-wide tiles without a K split for 75 .. 148 tiles of at most 32 k-blocks (64 elements each)
-@pytest.mark.parametrize("m,n,k", [(1, 72, 64), (7, 264, 200), (9, 264, 200), (63, 136, 72), (65, 136, 72), (121, 136, 72), (127, 64, 520), (5, 4736, 2048), (5, 4744, 2048),
-                                   (3, 9472, 2048), (3, 9480, 2048), (5, 4744, 2056)])
+# fetched rows come in groups of 8 (1 .. 128)
+@pytest.mark.parametrize("m,n,k", [(1, 72, 64), (7, 264, 200), (9, 264, 200), (63, 136, 72), (65, 136, 72), (121, 136, 72), (127, 64, 520), (5, 4744, 2056)])
 def test_few_rows(dev, orc, m, n, k):
     a = orc.round_bf16(orc.normal((m, k), 61))
     b = orc.round_bf16(orc.normal((n, k), 62))

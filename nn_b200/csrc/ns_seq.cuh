@@ -27,13 +27,22 @@ static inline bool ns_source_ok(uint64_t ptr, int splits, int dtype)
 
 #ifdef __CUDACC__
 
-// the value at element `idx` (row * ld + column); slabs are added in order
+// the value at element `idx` (row * ld + column); slabs are added in order.  The loads of up to seven slabs are issued together: one
+// after the other, each waiting for the sum before it, eight slabs cost eight round trips to L2.
 NS_DEVINL float ns_source_at(const NsSource& s, int64_t idx)
 {
     if (s.dtype == NS_BF16) return ns_bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(s.ptr)[idx]);
     const float* p = reinterpret_cast<const float*>(s.ptr) + idx;
     float v = p[0];
-    for (int i = 1; i < s.splits; i++) v = __fadd_rn(v, p[i * s.slab]);
+    for (int i = 1; i < s.splits; i += 7) {
+        float t[7];
+#pragma unroll
+        for (int j = 0; j < 7; j++)
+            if (i + j < s.splits) t[j] = p[(i + j) * s.slab];
+#pragma unroll
+        for (int j = 0; j < 7; j++)
+            if (i + j < s.splits) v = __fadd_rn(v, t[j]);
+    }
     return v;
 }
 // four consecutive values; idx and ld are multiples of 4 and ptr is 16-byte aligned
@@ -46,9 +55,16 @@ NS_DEVINL float4 ns_source_at4(const NsSource& s, int64_t idx)
     }
     const float* p = reinterpret_cast<const float*>(s.ptr) + idx;
     float4 v = *reinterpret_cast<const float4*>(p);
-    for (int i = 1; i < s.splits; i++) {
-        const float4 t = *reinterpret_cast<const float4*>(p + i * s.slab);
-        v.x = __fadd_rn(v.x, t.x); v.y = __fadd_rn(v.y, t.y); v.z = __fadd_rn(v.z, t.z); v.w = __fadd_rn(v.w, t.w);
+    for (int i = 1; i < s.splits; i += 7) {
+        float4 t[7];
+#pragma unroll
+        for (int j = 0; j < 7; j++)
+            if (i + j < s.splits) t[j] = *reinterpret_cast<const float4*>(p + (i + j) * s.slab);
+#pragma unroll
+        for (int j = 0; j < 7; j++)
+            if (i + j < s.splits) {
+                v.x = __fadd_rn(v.x, t[j].x); v.y = __fadd_rn(v.y, t[j].y); v.z = __fadd_rn(v.z, t[j].z); v.w = __fadd_rn(v.w, t[j].w);
+            }
     }
     return v;
 }

@@ -85,6 +85,9 @@ __global__ void __launch_bounds__(256) ns_rms_rows_kernel(const RmsArgs a)
     __shared__ float red[8];
     ns_pdl_wait();
     ns_pdl_trigger();
+    // asked for now, read after the reduction (see ns_rms_post_rows_vec_kernel)
+    if (VEC && a.w != nullptr)
+        for (int c = threadIdx.x * 32; c < a.cols; c += blockDim.x * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.w + c));
     const int row = a.row_map != nullptr ? a.row_map[blockIdx.x] : (int)blockIdx.x;
     const int64_t base = (int64_t)row * a.cols;
     float ss = 0.0f;
@@ -137,14 +140,26 @@ struct PostRmsArgs {
 template <typename T, int Q>
 __global__ void __launch_bounds__(256) ns_rms_post_rows_vec_kernel(const PostRmsArgs p)
 {
+    constexpr bool EARLY = Q <= 2;
     const RmsArgs& a = p.r;
     __shared__ float red[2][8];
     ns_pdl_wait();
     ns_pdl_trigger();
     const int row = blockIdx.x;
     const int64_t base = (int64_t)row * a.cols;
-    float4 s[Q], x[Q];
+    float4 s[Q], x[Q], pw[EARLY ? Q : 1], nw[EARLY ? Q : 1];
     float ss = 0.0f;
+    // A decoding step streams hundreds of megabytes of weights between two visits of these vectors, so each read of them is a trip
+    // to HBM: of a row short enough for the registers they are asked for together with the row, not after its two reductions.
+    if (EARLY) {
+#pragma unroll
+        for (int i = 0; i < Q; i++) {
+            const int c = (threadIdx.x + 256 * i) * 4;
+            if (c >= a.cols) continue;
+            pw[i] = __ldg(reinterpret_cast<const float4*>(p.post_w + c));
+            if (a.w != nullptr) nw[i] = __ldg(reinterpret_cast<const float4*>(a.w + c));
+        }
+    }
 #pragma unroll
     for (int i = 0; i < Q; i++) {
         const int c = (threadIdx.x + 256 * i) * 4;
@@ -165,7 +180,7 @@ __global__ void __launch_bounds__(256) ns_rms_post_rows_vec_kernel(const PostRms
     for (int i = 0; i < Q; i++) {
         const int c = (threadIdx.x + 256 * i) * 4;
         if (c >= a.cols) continue;
-        const float4 w = __ldg(reinterpret_cast<const float4*>(p.post_w + c));
+        const float4 w = EARLY ? pw[EARLY ? i : 0] : __ldg(reinterpret_cast<const float4*>(p.post_w + c));
         x[i] = make_float4(fmaf(s[i].x * post, w.x, x[i].x), fmaf(s[i].y * post, w.y, x[i].y), fmaf(s[i].z * post, w.z, x[i].z), fmaf(s[i].w * post, w.w, x[i].w));
         *reinterpret_cast<float4*>(a.x_out + base + c) = x[i];
         ss = fmaf(x[i].x, x[i].x, ss); ss = fmaf(x[i].y, x[i].y, ss); ss = fmaf(x[i].z, x[i].z, ss); ss = fmaf(x[i].w, x[i].w, ss);
@@ -177,7 +192,7 @@ __global__ void __launch_bounds__(256) ns_rms_post_rows_vec_kernel(const PostRms
     for (int i = 0; i < Q; i++) {
         const int c = (threadIdx.x + 256 * i) * 4;
         if (c >= a.cols) continue;
-        const float4 w = __ldg(reinterpret_cast<const float4*>(a.w + c));
+        const float4 w = EARLY ? nw[EARLY ? i : 0] : __ldg(reinterpret_cast<const float4*>(a.w + c));
         ns_store4(y + c, make_float4(x[i].x * inv * w.x, x[i].y * inv * w.y, x[i].z * inv * w.z, x[i].w * inv * w.w));
     }
     for (int c = a.cols + threadIdx.x; c < a.y_ld; c += blockDim.x) ns_store(y + c, 0.0f);

@@ -60,6 +60,31 @@ __device__ __forceinline__ int32_t sum_splits(const int32_t* __restrict__ partia
     return s;
 }
 
+// The same of eight consecutive elements (idx a multiple of 8).  The loads of four splits are issued together: a loop that adds one
+// split at a time pays an L2 round trip for each.
+__device__ __forceinline__ void sum_splits8(const int32_t* __restrict__ partial, int splits, size_t slab, size_t idx, int32_t (&acc)[8])
+{
+#pragma unroll
+    for (int i = 0; i < 8; i++) acc[i] = 0;
+    for (int sp = 0; sp < splits; sp += 4) {
+        int4 a[4], b[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            a[j] = b[j] = make_int4(0, 0, 0, 0);
+            if (sp + j < splits) {
+                const int4* src = reinterpret_cast<const int4*>(partial + (size_t)(sp + j) * slab + idx);
+                a[j] = src[0];
+                b[j] = src[1];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            acc[0] += a[j].x; acc[1] += a[j].y; acc[2] += a[j].z; acc[3] += a[j].w;
+            acc[4] += b[j].x; acc[5] += b[j].y; acc[6] += b[j].z; acc[7] += b[j].w;
+        }
+    }
+}
+
 struct FinishNormParams {
     const int32_t* partial;
     int splits;
@@ -131,6 +156,20 @@ __global__ void ns_finish_norm_quant_reg_kernel(const FinishNormParams p)
     ns_pdl_trigger();
     __shared__ ns_rows::RowShared sh;
     const size_t slab = (size_t)p.rows * p.cols;
+    // the vectors that are read after the sums: asked for now (a trip to HBM each, after a step's worth of weights)
+#pragma unroll
+    for (int j = 0; j < VPT; j++) {
+        const int col = ns_rows::vec_col(j);
+        if ((threadIdx.x & 3) != 0) break;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w_scale + col));
+        if (p.bias != nullptr) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.bias + col));
+        if (p.gamma != nullptr) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.gamma + col));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.beta + col));
+        }
+        if (p.residual != nullptr && (threadIdx.x & 7) == 0 && blockIdx.x < p.rows)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.residual + (size_t)blockIdx.x * p.cols + col));
+    }
     for (int64_t r = blockIdx.x; r < p.rows; r += gridDim.x) {
         const float a_scale = p.x_scale[r];
         float v[VPT * 8];
@@ -138,13 +177,8 @@ __global__ void ns_finish_norm_quant_reg_kernel(const FinishNormParams p)
         for (int j = 0; j < VPT; j++) {
             const int col = ns_rows::vec_col(j);
             const size_t idx = (size_t)r * p.cols + col;
-            int32_t acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            for (int sp = 0; sp < p.splits; sp++) {
-                const int4* src = reinterpret_cast<const int4*>(p.partial + (size_t)sp * slab + idx);
-                const int4 a = src[0], b = src[1];
-                acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
-                acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
-            }
+            int32_t acc[8];
+            sum_splits8(p.partial, p.splits, slab, idx, acc);
             const float4 w0 = __ldg(reinterpret_cast<const float4*>(p.w_scale + col)), w1 = __ldg(reinterpret_cast<const float4*>(p.w_scale + col + 4));
             const float ws[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
             float t[8];
@@ -206,13 +240,8 @@ __global__ void ns_finish_gelu_quant_kernel(const FinishGeluParams p)
         for (int j = 0; j < VPT; j++) {
             const int col = ns_rows::vec_col(j);
             const size_t idx = (size_t)r * p.cols + col;
-            int32_t acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            for (int sp = 0; sp < p.splits; sp++) {
-                const int4* src = reinterpret_cast<const int4*>(p.partial + (size_t)sp * slab + idx);
-                const int4 a = src[0], b = src[1];
-                acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
-                acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
-            }
+            int32_t acc[8];
+            sum_splits8(p.partial, p.splits, slab, idx, acc);
             const float4 w0 = __ldg(reinterpret_cast<const float4*>(p.w_scale + col)), w1 = __ldg(reinterpret_cast<const float4*>(p.w_scale + col + 4));
             const float4 b0 = __ldg(reinterpret_cast<const float4*>(p.bias + col)), b1 = __ldg(reinterpret_cast<const float4*>(p.bias + col + 4));
             const float ws[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
@@ -271,13 +300,8 @@ __global__ void ns_finish_kv_append_kernel(const FinishKvParams p)
         const int col0 = (int)(e % groups) * 8;
         const size_t idx0 = (size_t)row * cols + col0;
         const float a_scale = p.x_scale[row];
-        int32_t acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int sp = 0; sp < p.splits; sp++) {
-            const int4* src = reinterpret_cast<const int4*>(p.partial + (size_t)sp * slab + idx0);
-            const int4 a = src[0], b = src[1];
-            acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
-            acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
-        }
+        int32_t acc[8];
+        sum_splits8(p.partial, p.splits, slab, idx0, acc);
         uint32_t w[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {

@@ -256,6 +256,19 @@ NS_API int ns_f32_permute(ns_device_t dev, uint64_t x, uint64_t y, const int* ou
 /* [199] dst[dstOffset + r*dstStride + c] (+)= src[srcOffset + r*srcStride + c] */
 NS_API int ns_f32_copy2d(ns_device_t dev, uint64_t src, int64_t srcOffset, int srcStride, uint64_t dst, int64_t dstOffset, int dstStride,
                          int rows, int cols, int accumulate);
+/* One cached step of the float32 decoder with its operators in few launches; every output has the operators' bits.
+ * ns_f32_linear: y = residual + gelu(layernorm(x) * w + bias), each of layernorm (gamma, beta), bias, gelu and residual left out when 0 --
+ * [227], [129], [107] or [230], [95] in one launch (Layers/Attention.cs:201-211).  x is [m, k], w [k, n], n and k multiples of 4, k at most 4096.
+ * w must not be written by work still queued: it is fetched before the kernel in front has finished.  y must not overlap x or residual. */
+NS_API int ns_f32_linear(ns_device_t dev, uint64_t x, uint64_t gamma, uint64_t beta, float eps, uint64_t w, uint64_t bias, uint64_t residual, int gelu,
+                         uint64_t y, int m, int n, int k);
+/* One new position per sequence: head split, [238] for keys and values, scores, [224] with [235]'s mask, weighted values, heads merged
+ * (Layers/Attention.cs:46-118).  qkv is [batch, 3 heads dim], the caches [batch, heads, capacity, dim], y [batch, heads dim]. */
+NS_API int ns_f32_attention_step(ns_device_t dev, uint64_t qkv, uint64_t keys, uint64_t values, uint64_t position, uint64_t y, int batch, int heads,
+                                 int capacity, int dim, float scale);
+/* x[b, i, :] = table[ids[b, i], :] + positions[position + i, :] ([172] twice and the broadcast add of Layers/Attention.cs:268-269) */
+NS_API int ns_f32_embed_positions(ns_device_t dev, uint64_t ids, uint64_t table, uint64_t positions, uint64_t position, uint64_t x, int batch, int steps,
+                                  int dim, int vocabulary, int capacity);
 /* [248] SampleRows (kernel sample_rows_f32, Backends/Cuda/PtxKernels.Decoding.cs:170-350; CPU twin
  * Backends/Cpu/CpuBackend.Decoding.cs:114-245).  Row r reads logits[r * rowStride + rowOffset + j], j < vocabulary;
  * writes ids[r] (float-encoded) and 13 statistics at stats[(step[0] * rows + r) * 13]: id, probability, entropy in

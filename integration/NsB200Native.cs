@@ -273,6 +273,15 @@ internal static unsafe partial class NsB200Native
     public static partial int ns_f32_copy2d(nint dev, ulong src, long srcOffset, int srcStride, ulong dst, long dstOffset, int dstStride, int rows, int cols, int accumulate);
 
     [LibraryImport(Library)]
+    public static partial int ns_f32_linear(nint dev, ulong x, ulong gamma, ulong beta, float eps, ulong w, ulong bias, ulong residual, int gelu, ulong y, int m, int n, int k);
+
+    [LibraryImport(Library)]
+    public static partial int ns_f32_attention_step(nint dev, ulong qkv, ulong keys, ulong values, ulong position, ulong y, int batch, int heads, int capacity, int dim, float scale);
+
+    [LibraryImport(Library)]
+    public static partial int ns_f32_embed_positions(nint dev, ulong ids, ulong table, ulong positions, ulong position, ulong x, int batch, int steps, int dim, int vocabulary, int capacity);
+
+    [LibraryImport(Library)]
     public static partial int ns_f32_sample_rows(nint dev, ulong logits, ulong ids, ulong stats, ulong step, int rows, int vocabulary, int rowStride, int rowOffset, float temperature, int topK, float topP, float minP, uint seed);
 
     [LibraryImport(Library)]

@@ -1,20 +1,24 @@
-"""The reference's float32 decoder, operator for operator, on ``NsB200Backend``.
+"""The reference's float32 decoder on ``NsB200Backend``.
 
-This is the call sequence ``Sequential.ForwardCached`` issues for one cached step (src/NeuralSharp/Layers/
+A prompt is read operator for operator: this is the call sequence ``Sequential.ForwardCached`` issues for one cached step (src/NeuralSharp/Layers/
 Sequential.cs:59-80): Embedding (gather), PositionalEncoding.ForwardCached (gather + add), per layer LayerNorm
 (fused), the QKV Linear (product + AddRowVector), head split (Copy2D + Permute), KeyValueWrite, Q.K^T over the whole
 cache capacity, ScaleMaskSoftmax with the decoder mask, P.V, head merge (Permute), output Linear, residual Add,
 LayerNorm, product + BiasGelu, Linear, residual Add; then the final LayerNorm, the head and the greedy ArgMax of the
 last position.  Ids, the position and the sampled token are float-encoded values in device memory, as in the
-reference (Layers/Decoding.cs:69,81-82), so one recorded graph serves every position.
+reference (Layers/Decoding.cs:69,81-82), so one recorded graph serves every position.  A step of one position per sequence
+takes five launches a layer instead of 26, with the same bits (``_forward_step``), where the sizes allow it.
 
 It exists to show the operator surface is a drop-in (same results as the CPU backend on the same weights) and to run
 benchmark configuration 1; the fast path for large models is ``nn_b200.gpt.GptW8A8``.
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import numpy as np
 
+from . import native as N
 from .backend import NsB200Backend
 from .device import Device
 from .gpt import GptConfig
@@ -49,6 +53,8 @@ class GptF32:
         self.values = [a(batch * H * cap * dh, True) for _ in range(cfg.layers)]
         self.next_ids = a(batch, True)
         self.length = 0
+        # sizes the step kernels take: vectors of four floats, an input row of each product and a head's values in shared memory
+        self.step_kernels = D % 4 == 0 and FF % 4 == 0 and V % 4 == 0 and dh % 4 == 0 and max(D, FF) <= 4096 and (cap * dh + cap + dh) * 4 <= 200 * 1024
         self.graph = None
         self.sampler = None                         # a TokenSampler replaces the greedy choice (CharGpt.cs:283-300)
 
@@ -76,6 +82,8 @@ class GptF32:
         D, H, dh, FF, V, cap = cfg.dim, cfg.heads, cfg.head_dim, cfg.ff_dim, cfg.vocab, cfg.context
         t, m = steps, B * steps
         assert self.length + t <= cap and t <= self.max_steps, "DecodingContext.BeginStep: capacity exceeded"
+        if t == 1 and self.step_kernels:
+            return self._forward_step()
         # DecodingContext.BeginStep (Layers/Decoding.cs:94-118): mask and positions from the device-side position
         be.DecoderMask(self.position, self.mask, t, cap)
         be.Copy(self.iota, self.positions, t)
@@ -111,6 +119,33 @@ class GptF32:
         self.x, self.x2 = x, x2
         be.LayerNormFused(x, w["lnf_g"], w["lnf_b"], self.h, m, D, cfg.eps)
         self._linear(self.h, w["head_w"], w["head_b"], self.logits, m, D, V)
+        self._end_step(t)
+
+    def _forward_step(self) -> None:
+        """``forward(1)`` in five launches a layer: the products with the LayerNorm in front of them and the bias, GELU and residual behind them,
+        and one kernel for everything between the QKV product and the output projection."""
+        cfg, h, m, w = self.cfg, self.dev.handle, self.batch, self.w
+        D, H, dh, FF, V, cap = cfg.dim, cfg.heads, cfg.head_dim, cfg.ff_dim, cfg.vocab, cfg.context
+        eps, scale = C.c_float(cfg.eps), C.c_float(np.float32(1.0) / np.sqrt(np.float32(dh)))
+
+        def linear(x, norm, weight, bias, residual, gelu, y, n, k):
+            g, b = (w[norm + "_g"].ptr, w[norm + "_b"].ptr) if norm else (0, 0)
+            N.call("ns_f32_linear", h, x.ptr, g, b, eps, w[weight].ptr, w[bias].ptr, residual.ptr if residual else 0, gelu, y.ptr, m, n, k)
+
+        N.call("ns_f32_embed_positions", h, self.ids.ptr, w["tok"].ptr, w["pos"].ptr, self.position.ptr, self.x.ptr, m, 1, D, V, cap)
+        x, x2 = self.x, self.x2
+        for i in range(cfg.layers):
+            p = f"l{i}."
+            linear(x, p + "ln1", p + "qkv_w", p + "qkv_b", None, 0, self.qkv, 3 * D, D)
+            N.call("ns_f32_attention_step", h, self.qkv.ptr, self.keys[i].ptr, self.values[i].ptr, self.position.ptr, self.merged.ptr, m, H, cap, dh, scale)
+            linear(self.merged, None, p + "out_w", p + "out_b", x, 0, x2, D, D)
+            linear(x2, p + "ln2", p + "ff1_w", p + "ff1_b", None, 1, self.ffa, FF, D)
+            linear(self.ffa, None, p + "ff2_w", p + "ff2_b", x2, 0, x, D, FF)
+        linear(x, "lnf", "head_w", "head_b", None, 0, self.logits, V, D)
+        self._end_step(1)
+
+    def _end_step(self, t: int) -> None:
+        be, B, V = self.be, self.batch, self.cfg.vocab
         # greedy token of the last position (TokenSampler reads row r at r * rowStride + rowOffset, Sampling.cs:122)
         if self.sampler is None:
             be.ArgMaxRows(self.logits, self.next_ids, B, V, t * V, (t - 1) * V)

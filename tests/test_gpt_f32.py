@@ -6,9 +6,13 @@ GraphReplay (:144-189, graph == direct over 8 steps), and benchmark configuratio
 4 layers, 4 heads, FFN 512, context 128, prompt 32, greedy 128 tokens: logits <= 1e-4, token ids equal, one context
 reset at the 97th token).
 """
+import ctypes as C
+
 import numpy as np
 import pytest
 
+from nn_b200 import native as N
+from nn_b200.backend import NsB200Backend
 from nn_b200.gpt import GptConfig
 from nn_b200.gpt_f32 import GptF32
 from oracle import model as om
@@ -82,3 +86,49 @@ def test_baseline_config_1(dev, orc, sinusoid):
     if first_div is not None:
         top2 = np.sort(ref.logit_trace[first_div][0])[-2:]
         assert top2[1] - top2[0] <= 2e-4 * max(1.0, abs(top2[1])), f"tokens diverge at step {first_div} without a near-tie"
+
+
+# around a warp's rows (1, 2 and 4 of tiles of 8, 16 and 32), a tile's 32 columns, the ring's 64-step slices (8 of them), the longest row of each form
+@pytest.mark.parametrize("m,n,k", [(1, 4, 4), (1, 128, 512), (3, 36, 60), (8, 32, 64), (9, 28, 452), (17, 100, 516), (33, 64, 1024), (17, 32, 1028), (9, 8, 2052), (2, 8, 4096)])
+def test_step_linear_has_the_operators_bits(dev, orc, m, n, k):
+    be = NsB200Backend(dev)
+    up = lambda a: dev.from_numpy(np.ascontiguousarray(a, dtype=np.float32))
+    x, w, g, b, bias, res = (up(orc.normal(s, 80 + i)) for i, s in enumerate([(m, k), (k, n), (k,), (k,), (n,), (m, n)]))
+    y, t, u = dev.empty(m * n), dev.empty(m * k), dev.empty(m * n)
+    bits = lambda s: s.download(count=m * n).view(np.uint32)
+    for norm, with_bias, gelu, residual in [(0, 0, 0, 0), (1, 1, 0, 0), (1, 1, 1, 0), (0, 1, 0, 1), (1, 0, 0, 1)]:
+        N.call("ns_f32_linear", dev.handle, x.ptr, g.ptr if norm else 0, b.ptr if norm else 0, C.c_float(1e-5), w.ptr, bias.ptr if with_bias else 0,
+               res.ptr if residual else 0, gelu, y.ptr, m, n, k)
+        if norm:
+            be.LayerNormFused(x, g, b, t, m, k, 1e-5)
+        be.MatMul(t if norm else x, w, u, m, n, k, False, False, 0.0)
+        if gelu:
+            be.BiasGelu(u, bias, u, m * n, n)
+        elif with_bias:
+            be.AddRowVector(u, bias, u, m, n)
+        if residual:
+            be.Add(res, u, u, m * n)
+        dev.synchronize()
+        assert np.array_equal(bits(y), bits(u)), (norm, with_bias, gelu, residual)
+
+
+@pytest.mark.parametrize("batch,heads,cap,dim,pos", [(1, 4, 128, 32, 0), (2, 3, 128, 32, 127), (1, 2, 5, 4, 3), (3, 2, 300, 36, 129), (1, 2, 257, 132, 256), (1, 1, 12, 8, 12)])
+def test_step_attention_has_the_operators_bits(dev, orc, batch, heads, cap, dim, pos):
+    be, D = NsB200Backend(dev), heads * dim
+    up = lambda a: dev.from_numpy(np.ascontiguousarray(a, dtype=np.float32))
+    qkv_h, k_h, v_h = orc.normal((batch, 3 * D), 90), orc.normal((batch * heads, cap, dim), 91), orc.normal((batch * heads, cap, dim), 92)
+    qkv, position = up(qkv_h), up([float(pos)])
+    got, exp = [up(k_h), up(v_h), dev.empty(batch * D)], [up(k_h), up(v_h), dev.empty(batch * D)]
+    scale = float(np.float32(dim) ** np.float32(-0.5))
+    N.call("ns_f32_attention_step", dev.handle, qkv.ptr, got[0].ptr, got[1].ptr, position.ptr, got[2].ptr, batch, heads, cap, dim, C.c_float(scale))
+    part = [up(qkv_h[:, i * D:(i + 1) * D]) for i in range(3)]           # one position: [batch, heads, 1, dim] as it lies
+    mask, scores, probs = dev.empty(cap), dev.empty(batch * heads * cap), dev.empty(batch * heads * cap)
+    be.DecoderMask(position, mask, 1, cap)
+    be.KeyValueWrite(part[1], exp[0], position, batch * heads, 1, cap, dim)
+    be.KeyValueWrite(part[2], exp[1], position, batch * heads, 1, cap, dim)
+    be.BatchedMatMul(part[0], exp[0], scores, batch * heads, 1, cap, dim, False, True, 0.0)
+    be.ScaleMaskSoftmax(scores, mask, probs, batch * heads, cap, 1, scale)
+    be.BatchedMatMul(probs, exp[1], exp[2], batch * heads, 1, dim, cap, False, False, 0.0)
+    dev.synchronize()
+    for a, b in zip(got, exp):
+        assert np.array_equal(a.download().view(np.uint32), b.download().view(np.uint32))

@@ -182,3 +182,18 @@ def test_many_row_kernel_gives_up_when_a_copy_never_arrives(dev, orc):
     N.call("ns_quantize_rows_i8", dev.handle, dx.ptr, N.NS_BF16, C.c_int64(rows), cols, dq.ptr, ds.ptr)
     dev.synchronize()
     assert np.array_equal(dq.download((rows, cols)), q) and np.array_equal(ds.download(), sc)
+
+
+@pytest.mark.parametrize("batch,steps,dim", [(1, 1, 8), (3, 5, 24), (2, 3, 2048), (1, 3, 20)])
+def test_embed_pos_of_bf16_tables(dev, orc, batch, steps, dim):
+    """Eight columns a thread where dim allows it; ids and positions past the tables are clamped."""
+    V, ctx, p0 = 37, 6, 3
+    tok, pos = orc.round_bf16(orc.normal((V, dim), 71)), orc.round_bf16(orc.normal((ctx, dim), 72))
+    ids = np.random.default_rng(73).integers(-3, V + 3, (batch, steps)).astype(np.int32)
+    d = [dev.from_numpy(a) for a in (ids, tok, pos, np.array([p0], np.int32))]
+    y = dev.empty(batch * steps * dim, N.NS_BF16)
+    N.call("ns_embed_pos", dev.handle, d[0].ptr, d[1].ptr, d[2].ptr, N.NS_BF16, d[3].ptr, batch, steps, dim, V, ctx, N.NS_BF16, y.ptr)
+    dev.synchronize()
+    at = np.minimum(p0 + np.arange(steps), ctx - 1)
+    exp = orc.round_bf16(orc.widen_bf16(tok)[np.clip(ids, 0, V - 1)] + orc.widen_bf16(pos)[at][None])
+    assert np.array_equal(y.download((batch, steps, dim)), exp)

@@ -45,7 +45,10 @@ NS_DEVINL float ns_source_at(const NsSource& s, int64_t idx)
     }
     return v;
 }
-// four consecutive values; idx and ld are multiples of 4 and ptr is 16-byte aligned
+// four consecutive values; idx and ld are multiples of 4 and ptr is 16-byte aligned.  SLABS false: there is one slab.  Kernels that also
+// read a prompt's finished matrix are built both ways: the registers of seven slabs cost the many rows a third of their warps in
+// flight (8192 rows of 2048, residual + norm: 51.8 against 38.7 us).
+template <bool SLABS = true>
 NS_DEVINL float4 ns_source_at4(const NsSource& s, int64_t idx)
 {
     if (s.dtype == NS_BF16) {
@@ -55,7 +58,7 @@ NS_DEVINL float4 ns_source_at4(const NsSource& s, int64_t idx)
     }
     const float* p = reinterpret_cast<const float*>(s.ptr) + idx;
     float4 v = *reinterpret_cast<const float4*>(p);
-    for (int i = 1; i < s.splits; i += 7) {
+    for (int i = 1; SLABS && i < s.splits; i += 7) {
         float4 t[7];
 #pragma unroll
         for (int j = 0; j < 7; j++)

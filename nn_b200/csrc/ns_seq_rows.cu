@@ -77,7 +77,7 @@ struct RmsArgs {
     int64_t y_ld;
 };
 
-template <typename T, bool VEC>
+template <typename T, bool VEC, bool SLABS>
 __global__ void __launch_bounds__(256) ns_rms_rows_kernel(const RmsArgs a)
 {
     extern __shared__ float4 rms_row4[];
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(256) ns_rms_rows_kernel(const RmsArgs a)
     ns_pdl_wait();
     ns_pdl_trigger();
     // asked for now, read after the reduction (see ns_rms_post_rows_vec_kernel)
-    if (VEC && a.w != nullptr)
+    if (VEC && SLABS && a.w != nullptr)
         for (int c = threadIdx.x * 32; c < a.cols; c += blockDim.x * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.w + c));
     const int row = a.row_map != nullptr ? a.row_map[blockIdx.x] : (int)blockIdx.x;
     const int64_t base = (int64_t)row * a.cols;
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(256) ns_rms_rows_kernel(const RmsArgs a)
         for (int c = threadIdx.x * 4; c < a.cols; c += blockDim.x * 4) {
             float4 v = a.x != nullptr ? *reinterpret_cast<const float4*>(a.x + base + c) : make_float4(0.f, 0.f, 0.f, 0.f);
             if (a.src.ptr != nullptr) {
-                const float4 s = ns_source_at4(a.src, (int64_t)row * a.src.ld + c);
+                const float4 s = ns_source_at4<SLABS>(a.src, (int64_t)row * a.src.ld + c);
                 v.x = fmaf(a.alpha, s.x, v.x); v.y = fmaf(a.alpha, s.y, v.y); v.z = fmaf(a.alpha, s.z, v.z); v.w = fmaf(a.alpha, s.w, v.w);
             }
             if (a.x_out != nullptr) *reinterpret_cast<float4*>(a.x_out + base + c) = v;
@@ -137,10 +137,10 @@ struct PostRmsArgs {
 };
 
 // Q: groups of four columns a thread keeps in registers
-template <typename T, int Q>
+template <typename T, int Q, bool SLABS>
 __global__ void __launch_bounds__(256) ns_rms_post_rows_vec_kernel(const PostRmsArgs p)
 {
-    constexpr bool EARLY = Q <= 2;
+    constexpr bool EARLY = SLABS && Q <= 2;
     const RmsArgs& a = p.r;
     __shared__ float red[2][8];
     ns_pdl_wait();
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(256) ns_rms_post_rows_vec_kernel(const PostRms
         const int c = (threadIdx.x + 256 * i) * 4;
         s[i] = x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (c >= a.cols) continue;
-        s[i] = ns_source_at4(a.src, (int64_t)row * a.src.ld + c);
+        s[i] = ns_source_at4<SLABS>(a.src, (int64_t)row * a.src.ld + c);
         x[i] = *reinterpret_cast<const float4*>(a.x + base + c);
         if (p.plus != nullptr) {
             const float4 t = *reinterpret_cast<const float4*>(p.plus + base + c);
@@ -367,8 +367,8 @@ extern "C" int ns_rms_rows(ns_device_t h, uint64_t x, uint64_t src, int splits, 
         NS_CUDA(ns_launch_plain(kernel, dim3((unsigned)rows), dim3(256), smem, d->stream, a));
         return NS_OK;
     };
-    if (w == 0 || out_dtype == NS_F32) return vec ? launch(ns_rms_rows_kernel<float, true>) : launch(ns_rms_rows_kernel<float, false>);
-    return vec ? launch(ns_rms_rows_kernel<uint16_t, true>) : launch(ns_rms_rows_kernel<uint16_t, false>);
+    if (w == 0 || out_dtype == NS_F32) return !vec ? launch(ns_rms_rows_kernel<float, false, true>) : a.src.splits > 1 ? launch(ns_rms_rows_kernel<float, true, true>) : launch(ns_rms_rows_kernel<float, true, false>);
+    return !vec ? launch(ns_rms_rows_kernel<uint16_t, false, true>) : a.src.splits > 1 ? launch(ns_rms_rows_kernel<uint16_t, true, true>) : launch(ns_rms_rows_kernel<uint16_t, true, false>);
 }
 
 extern "C" int ns_rms_post_rows(ns_device_t h, uint64_t x, uint64_t src, int splits, int src_dtype, int src_ld, uint64_t post_w, uint64_t plus, uint64_t x_out, uint64_t w,
@@ -403,10 +403,10 @@ extern "C" int ns_rms_post_rows(ns_device_t h, uint64_t x, uint64_t src, int spl
     auto pick = [&](auto zero) -> int {
         using T = decltype(zero);
         if (!vec) return launch(ns_rms_post_rows_kernel<T>);
-        if (cols <= 1024) return launch(ns_rms_post_rows_vec_kernel<T, 1>);
-        if (cols <= 2048) return launch(ns_rms_post_rows_vec_kernel<T, 2>);
-        if (cols <= 4096) return launch(ns_rms_post_rows_vec_kernel<T, 4>);
-        return launch(ns_rms_post_rows_vec_kernel<T, 8>);
+        if (cols <= 1024) return (a.src.splits > 1 ? launch(ns_rms_post_rows_vec_kernel<T, 1, true>) : launch(ns_rms_post_rows_vec_kernel<T, 1, false>));
+        if (cols <= 2048) return (a.src.splits > 1 ? launch(ns_rms_post_rows_vec_kernel<T, 2, true>) : launch(ns_rms_post_rows_vec_kernel<T, 2, false>));
+        if (cols <= 4096) return (a.src.splits > 1 ? launch(ns_rms_post_rows_vec_kernel<T, 4, true>) : launch(ns_rms_post_rows_vec_kernel<T, 4, false>));
+        return (a.src.splits > 1 ? launch(ns_rms_post_rows_vec_kernel<T, 8, true>) : launch(ns_rms_post_rows_vec_kernel<T, 8, false>));
     };
     return w == 0 || out_dtype == NS_F32 ? pick(float(0)) : pick(uint16_t(0));
 }

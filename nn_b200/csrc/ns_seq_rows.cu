@@ -269,6 +269,43 @@ __global__ void __launch_bounds__(256) ns_glu_rows_kernel(const NsSource s, int6
     }
 }
 
+// The same of one finished bf16 matrix into bf16, eight columns a step and two steps in flight a thread (ff, both pitches multiples of 8, all on 16
+// bytes): the activations of a prompt.  Bound by HBM -- two values in, one out.  8192 x 5632, GELU: 78 -> 42 us (6.6 TB/s)
+// against four columns a step; ReLU 61 -> 39.
+template <int ACT>
+__global__ void __launch_bounds__(256) ns_glu_bf16_kernel(const uint16_t* src, int64_t ld, uint32_t n, uint32_t per_row, int ff, uint16_t* y, int64_t y_ld)
+{
+    ns_pdl_wait();
+    ns_pdl_trigger();
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t e0 = blockIdx.x * blockDim.x + threadIdx.x; e0 < n; e0 += 2 * stride) {
+        uint4 g[2], u[2];
+        int64_t at[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const uint32_t e = e0 + i * stride, r = e / per_row;
+            const int c = (int)(e - r * per_row) * 8;
+            at[i] = (int64_t)r * y_ld + c;
+            g[i] = u[i] = make_uint4(0, 0, 0, 0);
+            if (e >= n || c >= ff) continue;
+            const uint16_t* row = src + (int64_t)r * ld + c;
+            g[i] = *reinterpret_cast<const uint4*>(row);
+            u[i] = *reinterpret_cast<const uint4*>(row + ff);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            if (e0 + i * stride >= n) continue;
+            const uint32_t a[4] = {g[i].x, g[i].y, g[i].z, g[i].w}, b[4] = {u[i].x, u[i].y, u[i].z, u[i].w};
+            uint32_t o[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                o[j] = ns_pack_bf16x2(glu_act<uint16_t, ACT>(__uint_as_float(a[j] << 16)) * __uint_as_float(b[j] << 16),
+                                      glu_act<uint16_t, ACT>(__uint_as_float(a[j] & 0xFFFF0000u)) * __uint_as_float(b[j] & 0xFFFF0000u));
+            *reinterpret_cast<uint4*>(y + at[i]) = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+    }
+}
+
 // y[r, 0:cols] = source[r, col:col+cols], y[r, cols:y_ld] = 0
 template <typename T>
 __global__ void __launch_bounds__(256) ns_copy_cols_kernel(const NsSource s, int col, int64_t rows, int cols, T* __restrict__ y, int64_t y_ld)
@@ -428,6 +465,14 @@ extern "C" int ns_glu_rows(ns_device_t h, uint64_t src, int splits, int src_dtyp
     if (out_dtype == NS_F32) {
         if (act == NS_ACT_RELU) return vec ? launch(float(0), ns_glu_rows_kernel<float, true, NS_ACT_RELU>) : launch(float(0), ns_glu_rows_kernel<float, false, NS_ACT_RELU>);
         return vec ? launch(float(0), ns_glu_rows_kernel<float, true, NS_ACT_GELU>) : launch(float(0), ns_glu_rows_kernel<float, false, NS_ACT_GELU>);
+    }
+    const int64_t eights = rows * (int64_t)(y_ld / 8);
+    if (src_dtype == NS_BF16 && ((ff | src_ld | y_ld) & 7) == 0 && ((src | y) & 15) == 0 && eights < ((int64_t)1 << 31)) {
+        const dim3 blocks(flat_grid(d, (eights + 1) / 2));
+        auto kernel = act == NS_ACT_RELU ? ns_glu_bf16_kernel<NS_ACT_RELU> : ns_glu_bf16_kernel<NS_ACT_GELU>;
+        NS_CUDA(ns_launch_plain(kernel, blocks, dim3(256), 0, d->stream, reinterpret_cast<const uint16_t*>(src), (int64_t)src_ld, (uint32_t)eights, (uint32_t)(y_ld / 8), ff,
+                                reinterpret_cast<uint16_t*>(y), (int64_t)y_ld));
+        return NS_OK;
     }
     if (act == NS_ACT_RELU) return vec ? launch(uint16_t(0), ns_glu_rows_kernel<uint16_t, true, NS_ACT_RELU>) : launch(uint16_t(0), ns_glu_rows_kernel<uint16_t, false, NS_ACT_RELU>);
     return vec ? launch(uint16_t(0), ns_glu_rows_kernel<uint16_t, true, NS_ACT_GELU>) : launch(uint16_t(0), ns_glu_rows_kernel<uint16_t, false, NS_ACT_GELU>);

@@ -395,3 +395,16 @@ def test_bad_calls_are_refused(dev):
                 call(name, **bad)
     with pytest.raises(N.NsError):
         call("ns_window_prefill", vdim=20)                               # values that are no multiple of 8
+
+
+# around a thread's eight columns, two steps of the grid and a padded pitch; one matrix of bf16, both activations
+@pytest.mark.parametrize("rows,ff,ld,y_ld", [(1, 8, 16, 8), (3, 24, 56, 40), (257, 40, 80, 48), (2400, 5632, 11264, 5632)])
+def test_glu_of_a_bf16_matrix_is_that_of_its_float_values(dev, orc, rows, ff, ld, y_ld):
+    x = orc.round_bf16(orc.normal((rows, ld), 35, 2.0))
+    s16, s32 = dev.from_numpy(x), dev.from_numpy(orc.widen_bf16(x))
+    for act in (N.ACT_RELU, N.ACT_GELU):
+        got, exp = dev.empty(rows * y_ld, N.NS_BF16), dev.empty(rows * y_ld, N.NS_BF16)
+        N.call("ns_glu_rows", dev.handle, u(s16.ptr), 1, N.NS_BF16, ld, i64(rows), ff, act, N.NS_BF16, u(got.ptr), y_ld)
+        N.call("ns_glu_rows", dev.handle, u(s32.ptr), 1, N.NS_F32, ld, i64(rows), ff, act, N.NS_BF16, u(exp.ptr), y_ld)
+        dev.synchronize()
+        assert np.array_equal(got.download(), exp.download()), act

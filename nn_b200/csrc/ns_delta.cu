@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(256) ns_delta_recurrent_kernel(const DeltaArgs
 // ---------------------------------------------------------------------------------------------
 // y = o / sqrt(mean(o^2) + eps) * w * act(gate), per row and head
 // ---------------------------------------------------------------------------------------------
-template <typename T, bool VEC, bool SLABS>
+template <typename T, bool VEC, int SLABS>
 __global__ void __launch_bounds__(256) ns_gated_norm_kernel(const float* __restrict__ o, int o_ld, const NsSource gate, int gate_col, int act,
                                                             const float* __restrict__ w, float eps, int64_t rows, int heads, int vdim, T* __restrict__ y,
                                                             int64_t y_ld)
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(256) ns_gated_norm_kernel(const float* __restr
 }
 
 // The same for one wide head (the whole row): a CTA per row, up to 8 groups of four values per thread in registers.
-template <typename T, int Q, bool SLABS>
+template <typename T, int Q, int SLABS>
 __global__ void __launch_bounds__(256) ns_gated_norm_row_kernel(const float* __restrict__ o, int o_ld, const NsSource gate, int gate_col, int act,
                                                                 const float* __restrict__ w, float eps, int n, T* __restrict__ y, int64_t y_ld)
 {
@@ -615,20 +615,20 @@ extern "C" int ns_gated_norm(ns_device_t h, uint64_t o, int o_ld, uint64_t gate,
         };
         auto pick = [&](auto zero) -> int {
             using T = decltype(zero);
-            if (vdim <= 2048) return splits > 1 ? row(zero, ns_gated_norm_row_kernel<T, 2, true>) : row(zero, ns_gated_norm_row_kernel<T, 2, false>);
-            if (vdim <= 4096) return splits > 1 ? row(zero, ns_gated_norm_row_kernel<T, 4, true>) : row(zero, ns_gated_norm_row_kernel<T, 4, false>);
-            return splits > 1 ? row(zero, ns_gated_norm_row_kernel<T, 8, true>) : row(zero, ns_gated_norm_row_kernel<T, 8, false>);
+            if (vdim <= 2048) return splits > 1 ? row(zero, ns_gated_norm_row_kernel<T, 2, NS_TOGETHER>) : row(zero, ns_gated_norm_row_kernel<T, 2, NS_ONE_SLAB>);
+            if (vdim <= 4096) return splits > 1 ? row(zero, ns_gated_norm_row_kernel<T, 4, NS_TOGETHER>) : row(zero, ns_gated_norm_row_kernel<T, 4, NS_ONE_SLAB>);
+            return splits > 1 ? row(zero, ns_gated_norm_row_kernel<T, 8, NS_TOGETHER>) : row(zero, ns_gated_norm_row_kernel<T, 8, NS_ONE_SLAB>);
         };
         return out_dtype == NS_F32 ? pick(float(0)) : pick(uint16_t(0));
     }
     const int64_t blocks = (rows * heads + 7) / 8, most = (int64_t)d->sm_count * 32;
     const dim3 grid((unsigned)(blocks < most ? blocks : most));
     if (out_dtype == NS_F32) {
-        auto k = !vec ? ns_gated_norm_kernel<float, false, true> : splits > 1 ? ns_gated_norm_kernel<float, true, true> : ns_gated_norm_kernel<float, true, false>;
+        auto k = !vec ? ns_gated_norm_kernel<float, false, NS_TOGETHER> : splits > 1 ? ns_gated_norm_kernel<float, true, NS_TOGETHER> : ns_gated_norm_kernel<float, true, NS_ONE_SLAB>;
         NS_CUDA(ns_launch_plain(k, grid, dim3(256), 0, d->stream, reinterpret_cast<const float*>(o), o_ld, g, gate_col, act, reinterpret_cast<const float*>(w), eps,
                                 rows, heads, vdim, reinterpret_cast<float*>(y), (int64_t)y_ld));
     } else {
-        auto k = !vec ? ns_gated_norm_kernel<uint16_t, false, true> : splits > 1 ? ns_gated_norm_kernel<uint16_t, true, true> : ns_gated_norm_kernel<uint16_t, true, false>;
+        auto k = !vec ? ns_gated_norm_kernel<uint16_t, false, NS_TOGETHER> : splits > 1 ? ns_gated_norm_kernel<uint16_t, true, NS_TOGETHER> : ns_gated_norm_kernel<uint16_t, true, NS_ONE_SLAB>;
         NS_CUDA(ns_launch_plain(k, grid, dim3(256), 0, d->stream, reinterpret_cast<const float*>(o), o_ld, g, gate_col, act, reinterpret_cast<const float*>(w), eps,
                                 rows, heads, vdim, reinterpret_cast<uint16_t*>(y), (int64_t)y_ld));
     }

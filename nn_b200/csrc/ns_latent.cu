@@ -35,7 +35,7 @@ struct LatentAppendArgs {
     int ring_len, ring_ld;
 };
 
-template <typename T, bool VEC, bool SLABS>
+template <typename T, bool VEC, int SLABS>
 __global__ void __launch_bounds__(256) ns_latent_append_kernel(const LatentAppendArgs a)
 {
     extern __shared__ float4 app_smem[];
@@ -109,7 +109,7 @@ struct RotateArgs {
     void* rot; int64_t rot_ld; int rot_head;
 };
 
-template <typename TP, typename TR, bool VEC, bool SLABS>
+template <typename TP, typename TR, bool VEC, int SLABS>
 __global__ void __launch_bounds__(256) ns_rotate_heads_kernel(const RotateArgs a)
 {
     extern __shared__ float2 cs[];
@@ -354,8 +354,8 @@ extern "C" int ns_latent_append(ns_device_t h, uint64_t src, int splits, int src
     const int n = q_rank + kv_rank + rot_dim;
     NS_REQUIRE(n <= 12000, NS_ERR_ARGUMENT, "ns_latent_append: rows of %d values do not fit shared memory", n);
     const bool vec = ((q_rank | kv_rank | rot_dim | src_ld | cq_ld | ring_ld) & 3) == 0 && (ring_slot_stride & 3) == 0 && ((src | q_norm | kv_norm | cq | ring) & 15) == 0;
-    auto k = dtype == NS_F32 ? (!vec ? ns_latent_append_kernel<float, false, true> : splits > 1 ? ns_latent_append_kernel<float, true, true> : ns_latent_append_kernel<float, true, false>)
-                             : (!vec ? ns_latent_append_kernel<uint16_t, false, true> : splits > 1 ? ns_latent_append_kernel<uint16_t, true, true> : ns_latent_append_kernel<uint16_t, true, false>);
+    auto k = dtype == NS_F32 ? (!vec ? ns_latent_append_kernel<float, false, NS_TOGETHER> : splits > 1 ? ns_latent_append_kernel<float, true, NS_TOGETHER> : ns_latent_append_kernel<float, true, NS_ONE_SLAB>)
+                             : (!vec ? ns_latent_append_kernel<uint16_t, false, NS_TOGETHER> : splits > 1 ? ns_latent_append_kernel<uint16_t, true, NS_TOGETHER> : ns_latent_append_kernel<uint16_t, true, NS_ONE_SLAB>);
     NS_CUDA(ns_launch_plain(k, dim3((unsigned)(batch * steps)), dim3(256), (size_t)((n + 3) & ~3) * 4, d->stream, a));
     return NS_OK;
 }
@@ -382,9 +382,9 @@ extern "C" int ns_rotate_heads(ns_device_t h, uint64_t src, int splits, int src_
         NS_CUDA(ns_launch_plain(kern, dim3((unsigned)(batch * steps)), dim3(256), (size_t)(rot_dims / 2 + 1) * sizeof(float2), d->stream, a));
         return NS_OK;
     };
-    if (plain_dtype == NS_F32 && rot_dtype == NS_F32) return !vec ? go(ns_rotate_heads_kernel<float, float, false, true>) : splits > 1 ? go(ns_rotate_heads_kernel<float, float, true, true>) : go(ns_rotate_heads_kernel<float, float, true, false>);
+    if (plain_dtype == NS_F32 && rot_dtype == NS_F32) return !vec ? go(ns_rotate_heads_kernel<float, float, false, NS_TOGETHER>) : splits > 1 ? go(ns_rotate_heads_kernel<float, float, true, NS_TOGETHER>) : go(ns_rotate_heads_kernel<float, float, true, NS_ONE_SLAB>);
     if (plain_dtype == NS_BF16 && rot_dtype == NS_BF16)
-        return !vec ? go(ns_rotate_heads_kernel<uint16_t, uint16_t, false, true>) : splits > 1 ? go(ns_rotate_heads_kernel<uint16_t, uint16_t, true, true>) : go(ns_rotate_heads_kernel<uint16_t, uint16_t, true, false>);
+        return !vec ? go(ns_rotate_heads_kernel<uint16_t, uint16_t, false, NS_TOGETHER>) : splits > 1 ? go(ns_rotate_heads_kernel<uint16_t, uint16_t, true, NS_TOGETHER>) : go(ns_rotate_heads_kernel<uint16_t, uint16_t, true, NS_ONE_SLAB>);
     return ns_fail(NS_ERR_ARGUMENT, "ns_rotate_heads: both outputs have one type");
 }
 

@@ -173,7 +173,8 @@ NS_DEVINL float silu_fast(float z)
 
 // A tile [64, WIDTH] of the source from column `col` on, activated, as bf16 pairs: groups of four neighbouring channels, or of eight where the
 // source is one bf16 matrix (BF16).  Group x of a thread is element tid + THREADS x.  Rows past n and channels from `size` on are zero.
-// All loads are on their way before the first is used.
+// All loads of a finished matrix are on their way before the first is used.  Slabs are added one after the other: read together they spilled up
+// to 2 KB a thread (16 heads of 128 x 128, float: 200 tokens of one matrix 63.6 against 40.0 us, of four slabs 76.9 against 59.5).
 template <int WIDTH, int THREADS, bool BF16>
 struct Tile {
     static constexpr int PER = BF16 ? 8 : 4, GROUPS = WIDTH / PER, N = LC * GROUPS / THREADS > 0 ? LC * GROUPS / THREADS : 1;
@@ -202,12 +203,12 @@ struct Tile {
                 if (t >= n || t >= LC || c >= size) continue;
                 const int64_t at = (row0 + t) * s.ld + col + c;
                 if (vec) {
-                    f[i] = ns_source_at4(s, at);
+                    f[i] = ns_source_at4<NS_IN_TURN>(s, at);
                 } else {
-                    f[i].x = ns_source_at(s, at);
-                    if (c + 1 < size) f[i].y = ns_source_at(s, at + 1);
-                    if (c + 2 < size) f[i].z = ns_source_at(s, at + 2);
-                    if (c + 3 < size) f[i].w = ns_source_at(s, at + 3);
+                    f[i].x = ns_source_at<NS_IN_TURN>(s, at);
+                    if (c + 1 < size) f[i].y = ns_source_at<NS_IN_TURN>(s, at + 1);
+                    if (c + 2 < size) f[i].z = ns_source_at<NS_IN_TURN>(s, at + 2);
+                    if (c + 3 < size) f[i].w = ns_source_at<NS_IN_TURN>(s, at + 3);
                 }
             }
 #pragma unroll

@@ -27,28 +27,39 @@ static inline bool ns_source_ok(uint64_t ptr, int splits, int dtype)
 
 #ifdef __CUDACC__
 
-// the value at element `idx` (row * ld + column); slabs are added in order.  The loads of up to seven slabs are issued together: one
-// after the other, each waiting for the sum before it, eight slabs cost eight round trips to L2.
+// How a kernel adds up the slabs, always in order.  One after the other, each load waits for the sum before it: eight slabs cost eight
+// round trips to L2.  With the loads of seven slabs issued together it is one, but their registers cost warps in flight, and so
+// time wherever the rows are many: a kernel is built both ways, and its launch says where the line lies.
+//   NS_ONE_SLAB   there is one slab
+//   NS_IN_TURN    one after the other: finished matrices, two slabs (whose loads do not wait for each other either), many rows
+//   NS_TOGETHER   seven at a time: the many slabs of few rows
+constexpr int NS_ONE_SLAB = 0, NS_IN_TURN = 1, NS_TOGETHER = 7;
+
+// the value at element `idx` (row * ld + column)
+template <int SLABS = NS_TOGETHER>
 NS_DEVINL float ns_source_at(const NsSource& s, int64_t idx)
 {
     if (s.dtype == NS_BF16) return ns_bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(s.ptr)[idx]);
     const float* p = reinterpret_cast<const float*>(s.ptr) + idx;
     float v = p[0];
-    for (int i = 1; i < s.splits; i += 7) {
-        float t[7];
+    if constexpr (SLABS == NS_IN_TURN) {
+        for (int i = 1; i < s.splits; i++) v = __fadd_rn(v, p[i * s.slab]);
+    } else if constexpr (SLABS > 1) {
+        for (int i = 1; i < s.splits; i += SLABS) {
+            float t[SLABS];
 #pragma unroll
-        for (int j = 0; j < 7; j++)
-            if (i + j < s.splits) t[j] = p[(i + j) * s.slab];
+            for (int j = 0; j < SLABS; j++)
+                if (i + j < s.splits) t[j] = p[(i + j) * s.slab];
 #pragma unroll
-        for (int j = 0; j < 7; j++)
-            if (i + j < s.splits) v = __fadd_rn(v, t[j]);
+            for (int j = 0; j < SLABS; j++)
+                if (i + j < s.splits) v = __fadd_rn(v, t[j]);
+        }
     }
     return v;
 }
-// four consecutive values; idx and ld are multiples of 4 and ptr is 16-byte aligned.  SLABS false: there is one slab.  Kernels that also
-// read a prompt's finished matrix are built both ways: the registers of seven slabs cost the many rows a third of their warps in
-// flight (8192 rows of 2048, residual + norm: 51.8 against 38.7 us).
-template <bool SLABS = true>
+NS_DEVINL float4 ns_add4(float4 v, float4 t) { return make_float4(__fadd_rn(v.x, t.x), __fadd_rn(v.y, t.y), __fadd_rn(v.z, t.z), __fadd_rn(v.w, t.w)); }
+// four consecutive values; idx and ld are multiples of 4 and ptr is 16-byte aligned
+template <int SLABS = NS_TOGETHER>
 NS_DEVINL float4 ns_source_at4(const NsSource& s, int64_t idx)
 {
     if (s.dtype == NS_BF16) {
@@ -58,16 +69,18 @@ NS_DEVINL float4 ns_source_at4(const NsSource& s, int64_t idx)
     }
     const float* p = reinterpret_cast<const float*>(s.ptr) + idx;
     float4 v = *reinterpret_cast<const float4*>(p);
-    for (int i = 1; SLABS && i < s.splits; i += 7) {
-        float4 t[7];
+    if constexpr (SLABS == NS_IN_TURN) {
+        for (int i = 1; i < s.splits; i++) v = ns_add4(v, *reinterpret_cast<const float4*>(p + i * s.slab));
+    } else if constexpr (SLABS > 1) {
+        for (int i = 1; i < s.splits; i += SLABS) {
+            float4 t[SLABS];
 #pragma unroll
-        for (int j = 0; j < 7; j++)
-            if (i + j < s.splits) t[j] = *reinterpret_cast<const float4*>(p + (i + j) * s.slab);
+            for (int j = 0; j < SLABS; j++)
+                if (i + j < s.splits) t[j] = *reinterpret_cast<const float4*>(p + (i + j) * s.slab);
 #pragma unroll
-        for (int j = 0; j < 7; j++)
-            if (i + j < s.splits) {
-                v.x = __fadd_rn(v.x, t[j].x); v.y = __fadd_rn(v.y, t[j].y); v.z = __fadd_rn(v.z, t[j].z); v.w = __fadd_rn(v.w, t[j].w);
-            }
+            for (int j = 0; j < SLABS; j++)
+                if (i + j < s.splits) v = ns_add4(v, t[j]);
+        }
     }
     return v;
 }

@@ -77,7 +77,7 @@ struct RmsArgs {
     int64_t y_ld;
 };
 
-template <typename T, bool VEC, bool SLABS>
+template <typename T, bool VEC, int SLABS>
 __global__ void __launch_bounds__(256) ns_rms_rows_kernel(const RmsArgs a)
 {
     extern __shared__ float4 rms_row4[];
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(256) ns_rms_rows_kernel(const RmsArgs a)
     ns_pdl_wait();
     ns_pdl_trigger();
     // asked for now, read after the reduction (see ns_rms_post_rows_vec_kernel)
-    if (VEC && SLABS && a.w != nullptr)
+    if (VEC && SLABS != NS_ONE_SLAB && a.w != nullptr)
         for (int c = threadIdx.x * 32; c < a.cols; c += blockDim.x * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.w + c));
     const int row = a.row_map != nullptr ? a.row_map[blockIdx.x] : (int)blockIdx.x;
     const int64_t base = (int64_t)row * a.cols;
@@ -137,10 +137,10 @@ struct PostRmsArgs {
 };
 
 // Q: groups of four columns a thread keeps in registers
-template <typename T, int Q, bool SLABS>
+template <typename T, int Q, int SLABS>
 __global__ void __launch_bounds__(256) ns_rms_post_rows_vec_kernel(const PostRmsArgs p)
 {
-    constexpr bool EARLY = SLABS && Q <= 2;
+    constexpr bool EARLY = SLABS != NS_ONE_SLAB && Q <= 2;
     const RmsArgs& a = p.r;
     __shared__ float red[2][8];
     ns_pdl_wait();
@@ -404,8 +404,8 @@ extern "C" int ns_rms_rows(ns_device_t h, uint64_t x, uint64_t src, int splits, 
         NS_CUDA(ns_launch_plain(kernel, dim3((unsigned)rows), dim3(256), smem, d->stream, a));
         return NS_OK;
     };
-    if (w == 0 || out_dtype == NS_F32) return !vec ? launch(ns_rms_rows_kernel<float, false, true>) : a.src.splits > 1 ? launch(ns_rms_rows_kernel<float, true, true>) : launch(ns_rms_rows_kernel<float, true, false>);
-    return !vec ? launch(ns_rms_rows_kernel<uint16_t, false, true>) : a.src.splits > 1 ? launch(ns_rms_rows_kernel<uint16_t, true, true>) : launch(ns_rms_rows_kernel<uint16_t, true, false>);
+    if (w == 0 || out_dtype == NS_F32) return !vec ? launch(ns_rms_rows_kernel<float, false, NS_TOGETHER>) : a.src.splits > 1 ? launch(ns_rms_rows_kernel<float, true, NS_TOGETHER>) : launch(ns_rms_rows_kernel<float, true, NS_ONE_SLAB>);
+    return !vec ? launch(ns_rms_rows_kernel<uint16_t, false, NS_TOGETHER>) : a.src.splits > 1 ? launch(ns_rms_rows_kernel<uint16_t, true, NS_TOGETHER>) : launch(ns_rms_rows_kernel<uint16_t, true, NS_ONE_SLAB>);
 }
 
 extern "C" int ns_rms_post_rows(ns_device_t h, uint64_t x, uint64_t src, int splits, int src_dtype, int src_ld, uint64_t post_w, uint64_t plus, uint64_t x_out, uint64_t w,
@@ -440,10 +440,10 @@ extern "C" int ns_rms_post_rows(ns_device_t h, uint64_t x, uint64_t src, int spl
     auto pick = [&](auto zero) -> int {
         using T = decltype(zero);
         if (!vec) return launch(ns_rms_post_rows_kernel<T>);
-        if (cols <= 1024) return (a.src.splits > 1 ? launch(ns_rms_post_rows_vec_kernel<T, 1, true>) : launch(ns_rms_post_rows_vec_kernel<T, 1, false>));
-        if (cols <= 2048) return (a.src.splits > 1 ? launch(ns_rms_post_rows_vec_kernel<T, 2, true>) : launch(ns_rms_post_rows_vec_kernel<T, 2, false>));
-        if (cols <= 4096) return (a.src.splits > 1 ? launch(ns_rms_post_rows_vec_kernel<T, 4, true>) : launch(ns_rms_post_rows_vec_kernel<T, 4, false>));
-        return (a.src.splits > 1 ? launch(ns_rms_post_rows_vec_kernel<T, 8, true>) : launch(ns_rms_post_rows_vec_kernel<T, 8, false>));
+        if (cols <= 1024) return (a.src.splits > 1 ? launch(ns_rms_post_rows_vec_kernel<T, 1, NS_TOGETHER>) : launch(ns_rms_post_rows_vec_kernel<T, 1, NS_ONE_SLAB>));
+        if (cols <= 2048) return (a.src.splits > 1 ? launch(ns_rms_post_rows_vec_kernel<T, 2, NS_TOGETHER>) : launch(ns_rms_post_rows_vec_kernel<T, 2, NS_ONE_SLAB>));
+        if (cols <= 4096) return (a.src.splits > 1 ? launch(ns_rms_post_rows_vec_kernel<T, 4, NS_TOGETHER>) : launch(ns_rms_post_rows_vec_kernel<T, 4, NS_ONE_SLAB>));
+        return (a.src.splits > 1 ? launch(ns_rms_post_rows_vec_kernel<T, 8, NS_TOGETHER>) : launch(ns_rms_post_rows_vec_kernel<T, 8, NS_ONE_SLAB>));
     };
     return w == 0 || out_dtype == NS_F32 ? pick(float(0)) : pick(uint16_t(0));
 }

@@ -1,0 +1,40 @@
+"""Registers and spills of the kernels that read partial sums, as the compiler reports them (build/*.ptxas).  A kernel that holds the values of many
+slabs where a prompt has one finished matrix loses warps in flight, or spills, and no result shows it."""
+import os
+import re
+
+import pytest
+
+from nn_b200 import build
+
+if not os.path.exists(os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")):
+    pytest.skip("no nvcc", allow_module_level=True)
+
+
+@pytest.fixture(scope="module")
+def report():
+    """{mangled name: (registers, bytes spilled)}"""
+    build.make()
+    found = {}
+    for file in os.listdir(os.path.join(build.CSRC, "build")):
+        if file.endswith(".ptxas"):
+            text = open(os.path.join(build.CSRC, "build", file)).read()
+            for name, spill, regs in re.findall(r"Compiling entry function '(\S+)'.*?(\d+) bytes spill loads.*?Used (\d+) registers", text, re.S):
+                found[name] = (int(regs), int(spill))
+    return found
+
+
+# of every size the kernel is built for: registers that the smallest build may have (65536 a SM), bytes that any build may spill
+@pytest.mark.parametrize("kernel,most_registers,most_spilled", [
+    ("ns_lightning_chunk_kernel", 255, 32),
+])
+def test_kernels_of_many_rows_stay_small(report, kernel, most_registers, most_spilled):
+    builds = {n: v for n, v in report.items() if re.search(r"\d" + kernel + r"(I|E|v)", n)}
+    assert builds
+    # builds of one size differ in the last template argument, the number of slabs read together
+    sizes = {}
+    for name, (regs, spill) in builds.items():
+        assert spill <= most_spilled, (name, spill)
+        key = re.sub(r"Li\d+EE", "EE", name)
+        sizes[key] = min(regs, sizes.get(key, 1 << 30))
+    assert max(sizes.values()) <= most_registers, sizes

@@ -6,6 +6,8 @@
 // [rows, ld] of float or bf16.  NsSource describes either.
 #pragma once
 
+#include <type_traits>
+
 #include "ns_common.cuh"
 
 struct NsSource {
@@ -34,6 +36,13 @@ static inline bool ns_source_ok(uint64_t ptr, int splits, int dtype)
 //   NS_IN_TURN    one after the other: finished matrices, two slabs (whose loads do not wait for each other either), many rows
 //   NS_TOGETHER   seven at a time: the many slabs of few rows
 constexpr int NS_ONE_SLAB = 0, NS_IN_TURN = 1, NS_TOGETHER = 7;
+
+// f(the build that reads slabs together) or f(the build OTHER)
+template <int OTHER, typename F>
+static inline int ns_pick_slabs(bool together, F f)
+{
+    return together ? f(std::integral_constant<int, NS_TOGETHER>()) : f(std::integral_constant<int, OTHER>());
+}
 
 // the value at element `idx` (row * ld + column)
 template <int SLABS = NS_TOGETHER>

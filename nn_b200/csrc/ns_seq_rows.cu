@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(256) ns_rms_rows_kernel(const RmsArgs a)
     } else {
         for (int c = threadIdx.x; c < a.cols; c += blockDim.x) {
             float v = a.x != nullptr ? a.x[base + c] : 0.0f;
-            if (a.src.ptr != nullptr) v = fmaf(a.alpha, ns_source_at(a.src, (int64_t)row * a.src.ld + c), v);
+            if (a.src.ptr != nullptr) v = fmaf(a.alpha, ns_source_at<SLABS>(a.src, (int64_t)row * a.src.ld + c), v);
             if (a.x_out != nullptr) a.x_out[base + c] = v;
             ss = fmaf(v, v, ss);
             buf[c] = v;
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(256) ns_rms_post_rows_vec_kernel(const PostRms
     for (int c = a.cols + threadIdx.x; c < a.y_ld; c += blockDim.x) ns_store(y + c, 0.0f);
 }
 
-template <typename T>
+template <typename T, int SLABS>
 __global__ void __launch_bounds__(256) ns_rms_post_rows_kernel(const PostRmsArgs p)
 {
     const RmsArgs& a = p.r;
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(256) ns_rms_post_rows_kernel(const PostRmsArgs
     const int64_t base = (int64_t)row * a.cols;
     float ss = 0.0f;
     for (int c = threadIdx.x; c < a.cols; c += blockDim.x) {
-        buf[c] = ns_source_at(a.src, (int64_t)row * a.src.ld + c);
+        buf[c] = ns_source_at<SLABS>(a.src, (int64_t)row * a.src.ld + c);
         ss = fmaf(buf[c], buf[c], ss);
     }
     const float post = 1.0f / sqrtf(ns_cta_sum(ss, red[0]) / (float)a.cols + a.eps);
@@ -239,7 +239,7 @@ NS_DEVINL float glu_act(float g)
     return sizeof(T) == 2 ? ns_gelu_fast(g) : ns_gelu_tanh(g);
 }
 
-template <typename T, bool VEC, int ACT>
+template <typename T, bool VEC, int ACT, int SLABS>
 __global__ void __launch_bounds__(256) ns_glu_rows_kernel(const NsSource s, int64_t rows, int ff, T* __restrict__ y, int64_t y_ld)
 {
     ns_pdl_wait();
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(256) ns_glu_rows_kernel(const NsSource s, int6
             const int c = (int)(q - r * per_row) * 4;
             float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
             if (c < ff) {
-                const float4 g = ns_source_at4(s, r * s.ld + c), u = ns_source_at4(s, r * s.ld + ff + c);
+                const float4 g = ns_source_at4<SLABS>(s, r * s.ld + c), u = ns_source_at4<SLABS>(s, r * s.ld + ff + c);
                 o = make_float4(glu_act<T, ACT>(g.x) * u.x, glu_act<T, ACT>(g.y) * u.y, glu_act<T, ACT>(g.z) * u.z, glu_act<T, ACT>(g.w) * u.w);
             }
             ns_store4(y + r * y_ld + c, o);
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(256) ns_glu_rows_kernel(const NsSource s, int6
             const int64_t r = q / y_ld;
             const int c = (int)(q - r * y_ld);
             float o = 0.0f;
-            if (c < ff) o = glu_act<T, ACT>(ns_source_at(s, r * s.ld + c)) * ns_source_at(s, r * s.ld + ff + c);
+            if (c < ff) o = glu_act<T, ACT>(ns_source_at<SLABS>(s, r * s.ld + c)) * ns_source_at<SLABS>(s, r * s.ld + ff + c);
             ns_store(y + q, o);
         }
     }
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(256) ns_glu_bf16_kernel(const uint16_t* src, i
 }
 
 // y[r, 0:cols] = source[r, col:col+cols], y[r, cols:y_ld] = 0
-template <typename T>
+template <typename T, int SLABS>
 __global__ void __launch_bounds__(256) ns_copy_cols_kernel(const NsSource s, int col, int64_t rows, int cols, T* __restrict__ y, int64_t y_ld)
 {
     ns_pdl_wait();
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(256) ns_copy_cols_kernel(const NsSource s, int
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = q / y_ld;
         const int c = (int)(q - r * y_ld);
-        ns_store(y + q, c < cols ? ns_source_at(s, r * s.ld + col + c) : 0.0f);
+        ns_store(y + q, c < cols ? ns_source_at<SLABS>(s, r * s.ld + col + c) : 0.0f);
     }
 }
 
@@ -404,8 +404,12 @@ extern "C" int ns_rms_rows(ns_device_t h, uint64_t x, uint64_t src, int splits, 
         NS_CUDA(ns_launch_plain(kernel, dim3((unsigned)rows), dim3(256), smem, d->stream, a));
         return NS_OK;
     };
-    if (w == 0 || out_dtype == NS_F32) return !vec ? launch(ns_rms_rows_kernel<float, false, NS_TOGETHER>) : a.src.splits > 1 ? launch(ns_rms_rows_kernel<float, true, NS_TOGETHER>) : launch(ns_rms_rows_kernel<float, true, NS_ONE_SLAB>);
-    return !vec ? launch(ns_rms_rows_kernel<uint16_t, false, NS_TOGETHER>) : a.src.splits > 1 ? launch(ns_rms_rows_kernel<uint16_t, true, NS_TOGETHER>) : launch(ns_rms_rows_kernel<uint16_t, true, NS_ONE_SLAB>);
+    // 64 x 2047 of 8 slabs: 6.2 us together, 8.7 in turn; 8192 x 2047 of one slab: 83 in the build for many, 62 in its own
+    return ns_pick_slabs<NS_ONE_SLAB>(a.src.splits > 1, [&](auto slabs) {
+        constexpr int S = decltype(slabs)::value;
+        if (w == 0 || out_dtype == NS_F32) return vec ? launch(ns_rms_rows_kernel<float, true, S>) : launch(ns_rms_rows_kernel<float, false, S>);
+        return vec ? launch(ns_rms_rows_kernel<uint16_t, true, S>) : launch(ns_rms_rows_kernel<uint16_t, false, S>);
+    });
 }
 
 extern "C" int ns_rms_post_rows(ns_device_t h, uint64_t x, uint64_t src, int splits, int src_dtype, int src_ld, uint64_t post_w, uint64_t plus, uint64_t x_out, uint64_t w,
@@ -439,11 +443,13 @@ extern "C" int ns_rms_post_rows(ns_device_t h, uint64_t x, uint64_t src, int spl
     };
     auto pick = [&](auto zero) -> int {
         using T = decltype(zero);
-        if (!vec) return launch(ns_rms_post_rows_kernel<T>);
-        if (cols <= 1024) return (a.src.splits > 1 ? launch(ns_rms_post_rows_vec_kernel<T, 1, NS_TOGETHER>) : launch(ns_rms_post_rows_vec_kernel<T, 1, NS_ONE_SLAB>));
-        if (cols <= 2048) return (a.src.splits > 1 ? launch(ns_rms_post_rows_vec_kernel<T, 2, NS_TOGETHER>) : launch(ns_rms_post_rows_vec_kernel<T, 2, NS_ONE_SLAB>));
-        if (cols <= 4096) return (a.src.splits > 1 ? launch(ns_rms_post_rows_vec_kernel<T, 4, NS_TOGETHER>) : launch(ns_rms_post_rows_vec_kernel<T, 4, NS_ONE_SLAB>));
-        return (a.src.splits > 1 ? launch(ns_rms_post_rows_vec_kernel<T, 8, NS_TOGETHER>) : launch(ns_rms_post_rows_vec_kernel<T, 8, NS_ONE_SLAB>));
+        return ns_pick_slabs<NS_ONE_SLAB>(a.src.splits > 1, [&](auto slabs) {
+            constexpr int S = decltype(slabs)::value;
+            if (!vec) return launch(ns_rms_post_rows_kernel<T, S>);
+            if (cols <= 1024) return launch(ns_rms_post_rows_vec_kernel<T, 1, S>);
+            if (cols <= 2048) return launch(ns_rms_post_rows_vec_kernel<T, 2, S>);
+            return cols <= 4096 ? launch(ns_rms_post_rows_vec_kernel<T, 4, S>) : launch(ns_rms_post_rows_vec_kernel<T, 8, S>);
+        });
     };
     return w == 0 || out_dtype == NS_F32 ? pick(float(0)) : pick(uint16_t(0));
 }
@@ -457,25 +463,33 @@ extern "C" int ns_glu_rows(ns_device_t h, uint64_t src, int splits, int src_dtyp
     const NsSource s = ns_source(src, splits, src_dtype, rows, src_ld);
     const bool vec = ((ff | src_ld | y_ld) & 3) == 0 && ((src | y) & 15) == 0;
     const unsigned grid = flat_grid(d, vec ? rows * (y_ld / 4) : rows * y_ld);
+    // Slabs together (with vectors 96 registers, two CTAs a SM) where all CTAs are resident at once anyhow; without vectors (48 registers) also
+    // from five slabs on.  Together against in turn, 5632 columns, GELU to bf16 (us): 7 rows of 8 slabs 2.4, 3.0; 40 rows of 8 slabs
+    // 2.9, 3.3; 64 rows of 8 slabs 4.3, 3.7; 64 rows of 4 slabs 3.8, 2.9; 250 rows of 3 slabs 8.1, 4.8; 8192 rows 136, 83.  5631 columns:
+    // 64 rows of 8 slabs 4.9, 5.6; 250 rows of 3 slabs 12.5, 11.4; 8192 rows 220, 176.
+    const bool together = splits > 2 && (grid <= 2u * (unsigned)d->sm_count || (!vec && splits > 4));
     auto launch = [&](auto zero, auto kernel) -> int {
         using T = decltype(zero);
         NS_CUDA(ns_launch_plain(kernel, dim3(grid), dim3(256), 0, d->stream, s, rows, ff, reinterpret_cast<T*>(y), (int64_t)y_ld));
         return NS_OK;
     };
-    if (out_dtype == NS_F32) {
-        if (act == NS_ACT_RELU) return vec ? launch(float(0), ns_glu_rows_kernel<float, true, NS_ACT_RELU>) : launch(float(0), ns_glu_rows_kernel<float, false, NS_ACT_RELU>);
-        return vec ? launch(float(0), ns_glu_rows_kernel<float, true, NS_ACT_GELU>) : launch(float(0), ns_glu_rows_kernel<float, false, NS_ACT_GELU>);
-    }
     const int64_t eights = rows * (int64_t)(y_ld / 8);
-    if (src_dtype == NS_BF16 && ((ff | src_ld | y_ld) & 7) == 0 && ((src | y) & 15) == 0 && eights < ((int64_t)1 << 31)) {
+    if (out_dtype == NS_BF16 && src_dtype == NS_BF16 && ((ff | src_ld | y_ld) & 7) == 0 && ((src | y) & 15) == 0 && eights < ((int64_t)1 << 31)) {
         const dim3 blocks(flat_grid(d, (eights + 1) / 2));
         auto kernel = act == NS_ACT_RELU ? ns_glu_bf16_kernel<NS_ACT_RELU> : ns_glu_bf16_kernel<NS_ACT_GELU>;
         NS_CUDA(ns_launch_plain(kernel, blocks, dim3(256), 0, d->stream, reinterpret_cast<const uint16_t*>(src), (int64_t)src_ld, (uint32_t)eights, (uint32_t)(y_ld / 8), ff,
                                 reinterpret_cast<uint16_t*>(y), (int64_t)y_ld));
         return NS_OK;
     }
-    if (act == NS_ACT_RELU) return vec ? launch(uint16_t(0), ns_glu_rows_kernel<uint16_t, true, NS_ACT_RELU>) : launch(uint16_t(0), ns_glu_rows_kernel<uint16_t, false, NS_ACT_RELU>);
-    return vec ? launch(uint16_t(0), ns_glu_rows_kernel<uint16_t, true, NS_ACT_GELU>) : launch(uint16_t(0), ns_glu_rows_kernel<uint16_t, false, NS_ACT_GELU>);
+    auto pick = [&](auto zero) -> int {
+        using T = decltype(zero);
+        return ns_pick_slabs<NS_IN_TURN>(together, [&](auto slabs) {
+            constexpr int S = decltype(slabs)::value;
+            if (act == NS_ACT_RELU) return vec ? launch(zero, ns_glu_rows_kernel<T, true, NS_ACT_RELU, S>) : launch(zero, ns_glu_rows_kernel<T, false, NS_ACT_RELU, S>);
+            return vec ? launch(zero, ns_glu_rows_kernel<T, true, NS_ACT_GELU, S>) : launch(zero, ns_glu_rows_kernel<T, false, NS_ACT_GELU, S>);
+        });
+    };
+    return out_dtype == NS_F32 ? pick(float(0)) : pick(uint16_t(0));
 }
 
 extern "C" int ns_copy_cols(ns_device_t h, uint64_t src, int splits, int src_dtype, int src_ld, int col, int64_t rows, int cols, int out_dtype, uint64_t y,
@@ -486,12 +500,16 @@ extern "C" int ns_copy_cols(ns_device_t h, uint64_t src, int splits, int src_dty
     NS_REQUIRE(ns_source_ok(src, splits, src_dtype) && src_ld >= col + cols, NS_ERR_ARGUMENT, "ns_copy_cols: bad source");
     const NsSource s = ns_source(src, splits, src_dtype, rows, src_ld);
     const unsigned grid = flat_grid(d, rows * y_ld);
-    if (out_dtype == NS_F32)
-        NS_CUDA(ns_launch_plain(ns_copy_cols_kernel<float>, dim3(grid), dim3(256), 0, d->stream, s, col, rows, cols, reinterpret_cast<float*>(y), (int64_t)y_ld));
-    else
-        NS_CUDA(ns_launch_plain(ns_copy_cols_kernel<uint16_t>, dim3(grid), dim3(256), 0, d->stream, s, col, rows, cols, reinterpret_cast<uint16_t*>(y),
-                                (int64_t)y_ld));
-    return NS_OK;
+    // together against in turn (us): 64 x 2048, 8 slabs 2.1, 2.4; 250 x 2048, 3 slabs 4.3, 3.8; 8192 x 2048, one slab 60, 47
+    return ns_pick_slabs<NS_IN_TURN>(splits > 4, [&](auto slabs) -> int {
+        constexpr int S = decltype(slabs)::value;
+        if (out_dtype == NS_F32)
+            NS_CUDA(ns_launch_plain(ns_copy_cols_kernel<float, S>, dim3(grid), dim3(256), 0, d->stream, s, col, rows, cols, reinterpret_cast<float*>(y), (int64_t)y_ld));
+        else
+            NS_CUDA(ns_launch_plain(ns_copy_cols_kernel<uint16_t, S>, dim3(grid), dim3(256), 0, d->stream, s, col, rows, cols, reinterpret_cast<uint16_t*>(y),
+                                    (int64_t)y_ld));
+        return NS_OK;
+    });
 }
 
 extern "C" int ns_seq_advance(ns_device_t h, uint64_t ids, uint64_t slots, int batch, int steps, uint64_t pos, uint64_t last)

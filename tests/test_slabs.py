@@ -1,0 +1,76 @@
+"""Operators that read partial sums: whatever the number of slabs and however they are read, the bits are those of one slab that holds their
+sum in order.  Widths with and without vectors, few rows and many, up to one group of slabs read together (8) and past it."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from nn_b200 import native as N
+from tests.test_fabezen_ops import rng_for
+
+pytestmark = pytest.mark.gpu
+u, i64, fl = C.c_uint64, C.c_int64, C.c_float
+
+
+def slabs_and_sum(dev, rows, ld, splits):
+    parts = rng_for(splits, rows, ld).standard_normal((splits, rows, ld)).astype(np.float32)
+    total = parts[0].copy()
+    for p in parts[1:]:
+        total += p
+    return dev.from_numpy(parts), dev.from_numpy(total)
+
+
+def same(dev, run, source, total, splits):
+    """run(source, splits) returns what the operator wrote."""
+    got, want = run(source, splits), run(total, 1)
+    dev.synchronize()
+    for g, w in zip(got, want):
+        a, b = g.download(), w.download()
+        assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
+        assert np.any(a)
+
+
+SPLITS = [2, 3, 7, 8, 9, 16]
+
+
+@pytest.mark.parametrize("splits", SPLITS)
+@pytest.mark.parametrize("rows,cols", [(3, 64), (2, 61), (5, 1028), (300, 2048), (300, 2047), (3, 4096), (2, 8000), (2, 9001)])
+@pytest.mark.parametrize("out", [N.NS_F32, N.NS_BF16])
+def test_rows(dev, rows, cols, splits, out):
+    ld = (cols + 7) // 8 * 8
+    source, total = slabs_and_sum(dev, rows, ld, splits)
+    rng = rng_for(1, rows, cols)
+    x, w, post = (dev.from_numpy(rng.standard_normal(s).astype(np.float32)) for s in ((rows, cols), cols, cols))
+
+    def norm(src, n):
+        y, xo = dev.zeros(rows * ld, out), dev.zeros(rows * cols)
+        N.call("ns_rms_rows", dev.handle, u(x.ptr), u(src.ptr), n, N.NS_F32, ld, fl(0.3), u(xo.ptr), u(w.ptr), fl(1e-3), u(0), i64(rows), i64(rows), cols, out, u(y.ptr), ld)
+        return xo, y
+
+    def both_norms(src, n):
+        y, xo = dev.zeros(rows * ld, out), dev.zeros(rows * cols)
+        N.call("ns_rms_post_rows", dev.handle, u(x.ptr), u(src.ptr), n, N.NS_F32, ld, u(post.ptr), u(0), u(xo.ptr), u(w.ptr), fl(1e-3), i64(rows), cols, out, u(y.ptr), ld)
+        return xo, y
+
+    def columns(src, n):
+        y = dev.zeros(rows * ld, out)
+        N.call("ns_copy_cols", dev.handle, u(src.ptr), n, N.NS_F32, ld, 1, i64(rows), cols - 1, out, u(y.ptr), ld)
+        return (y,)
+
+    for run in (norm, both_norms, columns):
+        same(dev, run, source, total, splits)
+
+
+@pytest.mark.parametrize("splits", SPLITS)
+@pytest.mark.parametrize("rows,ff", [(1, 8), (3, 37), (3, 1000), (120, 5632), (60, 2047)])
+def test_gated_unit(dev, rows, ff, splits):
+    ld, y_ld = (2 * ff + 7) // 8 * 8, (ff + 7) // 8 * 8
+    source, total = slabs_and_sum(dev, rows, ld, splits)
+    for act in (N.ACT_GELU, N.ACT_RELU):
+        for out in (N.NS_F32, N.NS_BF16):
+            def unit(src, n):
+                y = dev.zeros(rows * y_ld, out)
+                N.call("ns_glu_rows", dev.handle, u(src.ptr), n, N.NS_F32, ld, i64(rows), ff, act, out, u(y.ptr), y_ld)
+                return (y,)
+
+            same(dev, unit, source, total, splits)

@@ -47,7 +47,7 @@ struct AppendArgs {
     Rings r;
 };
 
-template <typename T, bool VEC>
+template <typename T, bool VEC, int SLABS>
 __global__ void __launch_bounds__(256) ns_window_append_kernel(const AppendArgs a)
 {
     extern __shared__ float4 wa_smem[];
@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(256) ns_window_append_kernel(const AppendArgs 
     if (VEC) {
         for (int c = tid * 4; c < nq + nk; c += 1024) {
             const bool query = c < nq;
-            const float4 t = ns_source_at4(a.src, base + (query ? a.q_col + c : a.k_col + c - nq));
+            const float4 t = ns_source_at4<SLABS>(a.src, base + (query ? a.q_col + c : a.k_col + c - nq));
             *reinterpret_cast<float4*>(x + c) = t;
             const float s = fmaf(t.x, t.x, fmaf(t.y, t.y, fmaf(t.z, t.z, t.w * t.w)));
             if (query) sq += s;
@@ -75,23 +75,23 @@ __global__ void __launch_bounds__(256) ns_window_append_kernel(const AppendArgs 
         }
         for (int c = tid * 4; c < nv; c += 1024) {
             const int head = c / a.vdim;
-            ns_store4(v + head * v_head + c - head * a.vdim, ns_source_at4(a.src, base + a.v_col + c));
+            ns_store4(v + head * v_head + c - head * a.vdim, ns_source_at4<SLABS>(a.src, base + a.v_col + c));
         }
     } else {
         for (int c = tid; c < nq + nk; c += 256) {
             const bool query = c < nq;
-            const float t = ns_source_at(a.src, base + (query ? a.q_col + c : a.k_col + c - nq));
+            const float t = ns_source_at<SLABS>(a.src, base + (query ? a.q_col + c : a.k_col + c - nq));
             x[c] = t;
             if (query) sq = fmaf(t, t, sq);
             else sk = fmaf(t, t, sk);
         }
         for (int c = tid; c < nv; c += 256) {
             const int head = c / a.vdim;
-            ns_store(v + head * v_head + c - head * a.vdim, ns_source_at(a.src, base + a.v_col + c));
+            ns_store(v + head * v_head + c - head * a.vdim, ns_source_at<SLABS>(a.src, base + a.v_col + c));
         }
     }
     if (a.gate != nullptr)
-        for (int c = tid; c < a.heads; c += 256) a.gate[(int64_t)row * a.heads + c] = ns_sigmoid(ns_source_at(a.src, base + a.g_col + c));
+        for (int c = tid; c < a.heads; c += 256) a.gate[(int64_t)row * a.heads + c] = ns_sigmoid(ns_source_at<SLABS>(a.src, base + a.g_col + c));
     const float fq = 1.0f / sqrtf(ns_cta_sum(sq, red[0]) / (float)nq + a.eps);
     const float fk = 1.0f / sqrtf(ns_cta_sum(sk, red[1]) / (float)nk + a.eps);
     if (VEC) {
@@ -634,11 +634,18 @@ extern "C" int ns_window_append(ns_device_t h, uint64_t src, int splits, int src
     const size_t smem = ((size_t)(heads + kv_heads) * dim + 3) / 4 * 16;
     NS_REQUIRE(smem <= 200 * 1024, NS_ERR_ARGUMENT, "ns_window_append: queries and keys of %zu bytes do not fit shared memory", smem);
     const bool vec = ((dim | vdim | q_col | k_col | v_col | src_ld) & 3) == 0 && ((src | q_norm | k_norm | q) & 15) == 0 && (a.src.slab & 3) == 0;
-    auto k = dtype == NS_F32 ? (vec ? ns_window_append_kernel<float, true> : ns_window_append_kernel<float, false>)
-                             : (vec ? ns_window_append_kernel<uint16_t, true> : ns_window_append_kernel<uint16_t, false>);
-    if (smem > 48 * 1024) NS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    NS_CUDA(ns_launch_plain(k, dim3((unsigned)(batch * steps)), dim3(256), smem, d->stream, a));
-    return NS_OK;
+    auto go = [&](auto k) -> int {
+        if (smem > 48 * 1024) NS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        NS_CUDA(ns_launch_plain(k, dim3((unsigned)(batch * steps)), dim3(256), smem, d->stream, a));
+        return NS_OK;
+    };
+    // Together against in turn (us), 16 heads over 4 of 128 in vectors: 64 rows of 8 slabs 5.7, 7.3; of 4 slabs 5.4, 6.2; 200 rows of 2 slabs 5.8, 5.5;
+    // 16000 rows of one 154, 132.  15 over 3 heads of 33, value by value: 200 rows of 2 slabs 5.5, 5.9; 16000 rows of one 96, 89.
+    return ns_pick_slabs<NS_IN_TURN>(splits > (vec ? 2 : 1), [&](auto slabs) {
+        constexpr int S = decltype(slabs)::value;
+        if (dtype == NS_F32) return vec ? go(ns_window_append_kernel<float, true, S>) : go(ns_window_append_kernel<float, false, S>);
+        return vec ? go(ns_window_append_kernel<uint16_t, true, S>) : go(ns_window_append_kernel<uint16_t, false, S>);
+    });
 }
 
 extern "C" int ns_window_attend(ns_device_t h, int dtype, uint64_t q, uint64_t k_ring, uint64_t v_ring, int64_t k_slot_stride, int64_t v_slot_stride, int ring_len,

@@ -74,3 +74,22 @@ def test_gated_unit(dev, rows, ff, splits):
                 return (y,)
 
             same(dev, unit, source, total, splits)
+
+
+@pytest.mark.parametrize("splits", SPLITS)
+@pytest.mark.parametrize("H,G,dim,vdim,steps", [(4, 2, 32, 24, 3), (3, 1, 33, 27, 2), (16, 4, 128, 128, 70)])
+def test_window_append(dev, H, G, dim, vdim, steps, splits):
+    nq, nk, nv, ring = H * dim, G * dim, G * vdim, 128
+    k_ld, v_ld, rows = (dim + 7) // 8 * 8, (vdim + 7) // 8 * 8, 2 * steps
+    ld = (nq + nk + nv + H + 7) // 8 * 8
+    source, total = slabs_and_sum(dev, rows, ld, splits)
+    wq, wk = (dev.from_numpy(rng_for(3, n).standard_normal(n).astype(np.float32)) for n in (nq, nk))
+    slots, pos = dev.from_numpy(np.array([1, 0], np.int32)), dev.from_numpy(np.array([5, 90], np.int32))
+    for dtype in (N.NS_F32, N.NS_BF16):
+        def append(src, n):
+            q, gate, kr, vr = dev.zeros(rows * H * k_ld, dtype), dev.zeros(rows * H), dev.zeros(2 * G * ring * k_ld, dtype), dev.zeros(2 * G * ring * v_ld, dtype)
+            N.call("ns_window_append", dev.handle, u(src.ptr), n, N.NS_F32, ld, 0, nq, nq + nk, nq + nk + nv, H, G, dim, vdim, u(wq.ptr), u(wk.ptr), fl(1e-5), u(slots.ptr),
+                   u(pos.ptr), 2, steps, dtype, u(q.ptr), u(gate.ptr), u(kr.ptr), u(vr.ptr), i64(G * ring * k_ld), i64(G * ring * v_ld), ring, k_ld, v_ld)
+            return q, gate, kr, vr
+
+        same(dev, append, source, total, splits)

@@ -48,7 +48,7 @@ struct ConvArgs {
 // CTA share a head: 4 for prompts, 1 for the few tokens of a decoding step (the CTA then holds four heads).
 constexpr int CONV_WARP = 8;
 
-enum { CONV_ANY = 0, CONV_F32 = 1, CONV_BF16 = 2 };   // what the source is: anything, one float matrix, one bf16 matrix
+enum { CONV_ANY = 0, CONV_F32 = 1, CONV_BF16 = 2, CONV_SLABS = 3 };   // what the source is: anything, one float matrix, one bf16 matrix, many slabs
 
 template <int V, int SRC>
 NS_DEVINL void conv_load(const NsSource& s, int64_t idx, float (&x)[V])
@@ -61,15 +61,15 @@ NS_DEVINL void conv_load(const NsSource& s, int64_t idx, float (&x)[V])
         x[0] = __uint_as_float(w.x << 16); x[1] = __uint_as_float(w.x & 0xFFFF0000u);
         x[2] = __uint_as_float(w.y << 16); x[3] = __uint_as_float(w.y & 0xFFFF0000u);
     } else if constexpr (V == 4) {
-        const float4 t = ns_source_at4(s, idx);
+        const float4 t = ns_source_at4<SRC == CONV_SLABS ? NS_TOGETHER : NS_IN_TURN>(s, idx);
         x[0] = t.x; x[1] = t.y; x[2] = t.z; x[3] = t.w;
     } else {
 #pragma unroll
-        for (int i = 0; i < V; i++) x[i] = ns_source_at(s, idx + i);
+        for (int i = 0; i < V; i++) x[i] = ns_source_at<SRC == CONV_SLABS ? NS_TOGETHER : NS_IN_TURN>(s, idx + i);
     }
 }
 
-template <typename T, int V, int TAPS, int SRC = CONV_ANY>
+template <typename T, int V, int TAPS, int SRC>
 __global__ void __launch_bounds__(128) ns_short_conv_slide_kernel(const ConvArgs a, int span, int units, int pieces)
 {
     ns_pdl_wait();
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(128) ns_short_conv_slide_kernel(const ConvArgs
     }
 }
 
-template <typename T, int NV>
+template <typename T, int NV, int SLABS>
 __global__ void __launch_bounds__(128) ns_short_conv_kernel(const ConvArgs a)
 {
     ns_pdl_wait();
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(128) ns_short_conv_kernel(const ConvArgs a)
                 for (int n = 0; n < taps; n++) {
                     const int back = taps - 1 - n, tt = t - back;
                     float x = 0.0f;
-                    if (tt >= 0) x = ns_source_at(a.src, ((int64_t)b * a.steps + tt) * a.src.ld + g.col + c0 + c);
+                    if (tt >= 0) x = ns_source_at<SLABS>(a.src, ((int64_t)b * a.steps + tt) * a.src.ld + g.col + c0 + c);
                     else if (pos0 + tt >= 0) x = hist[(int64_t)((pos0 + tt) % taps) * channels + c0 + c];
                     acc = fmaf(x, __ldg(g.w + (int64_t)(c0 + c) * taps + n), acc);
                 }
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(128) ns_short_conv_kernel(const ConvArgs a)
     __syncthreads();
     for (int t = max(0, a.steps - (taps - 1)); t < a.steps; t++)
         for (int c = threadIdx.x; c < g.hd; c += blockDim.x)
-            hist[(int64_t)((pos0 + t) % taps) * channels + c0 + c] = ns_source_at(a.src, ((int64_t)b * a.steps + t) * a.src.ld + g.col + c0 + c);
+            hist[(int64_t)((pos0 + t) % taps) * channels + c0 + c] = ns_source_at<SLABS>(a.src, ((int64_t)b * a.steps + t) * a.src.ld + g.col + c0 + c);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -546,24 +546,35 @@ extern "C" int ns_short_conv(ns_device_t h, uint64_t src, int splits, int src_dt
             NS_CUDA(ns_launch_plain(k, sgrid, dim3(128), 0, d->stream, a, span, units, pieces));
             return NS_OK;
         };
+        // Slabs together, except where four channels a lane of four taps (146 registers against 128: three CTAs a SM, not four) need a second wave.
+        // Together against in turn (us): 32 heads of 128, 4 taps, 7 tokens of 8 slabs 3.9, 4.2; 64 of 4 slabs 9.0, 6.2; 250 of 4 slabs
+        // 12.4, 14.1; 6 taps, 64 tokens of 4 slabs 9.6, 10.1, 4 x 1000 tokens of one 106, 83; heads of 64, 4 taps, 64 of 4 slabs
+        // 4.6, 4.8, 4 x 1000 of one 36, 25.
+        const bool together = splits > 2 && (v < 4 || most_taps > 4 || (int64_t)sgrid.x * sgrid.y * sgrid.z <= 2 * d->sm_count);
         auto pick = [&](auto zero) -> int {
             using T = decltype(zero);
             if (v == 4 && most_taps <= 4 && splits == 1 && steps > CONV_WARP)
                 return src_dtype == NS_F32 ? slide(ns_short_conv_slide_kernel<T, 4, 4, CONV_F32>) : slide(ns_short_conv_slide_kernel<T, 4, 4, CONV_BF16>);
-            if (most_taps <= 4)
-                return v == 1 ? slide(ns_short_conv_slide_kernel<T, 1, 4>) : (v == 2 ? slide(ns_short_conv_slide_kernel<T, 2, 4>) : slide(ns_short_conv_slide_kernel<T, 4, 4>));
-            return v == 1 ? slide(ns_short_conv_slide_kernel<T, 1, 8>) : (v == 2 ? slide(ns_short_conv_slide_kernel<T, 2, 8>) : slide(ns_short_conv_slide_kernel<T, 4, 8>));
+            auto any = [&](auto source) -> int {
+                constexpr int S = decltype(source)::value;
+                if (most_taps <= 4)
+                    return v == 1 ? slide(ns_short_conv_slide_kernel<T, 1, 4, S>) : (v == 2 ? slide(ns_short_conv_slide_kernel<T, 2, 4, S>) : slide(ns_short_conv_slide_kernel<T, 4, 4, S>));
+                return v == 1 ? slide(ns_short_conv_slide_kernel<T, 1, 8, S>) : (v == 2 ? slide(ns_short_conv_slide_kernel<T, 2, 8, S>) : slide(ns_short_conv_slide_kernel<T, 4, 8, S>));
+            };
+            return together ? any(std::integral_constant<int, CONV_SLABS>()) : any(std::integral_constant<int, CONV_ANY>());
         };
         return out_dtype == NS_F32 ? pick(float(0)) : pick(uint16_t(0));
     }
-    if (out_dtype == NS_F32) {
-        if (widest <= 64) return launch(ns_short_conv_kernel<float, 2>);
-        if (widest <= 128) return launch(ns_short_conv_kernel<float, 4>);
-        return launch(ns_short_conv_kernel<float, 16>);
-    }
-    if (widest <= 64) return launch(ns_short_conv_kernel<uint16_t, 2>);
-    if (widest <= 128) return launch(ns_short_conv_kernel<uint16_t, 4>);
-    return launch(ns_short_conv_kernel<uint16_t, 16>);
+    // together against in turn (us): 8 heads of 256, 64 tokens of 4 slabs 14.0, 17.4; 8 of 100, 12 taps, 200 tokens of 2 slabs 64, 54; 4 x 1000 of one 97, 92
+    return ns_pick_slabs<NS_IN_TURN>(splits > 2, [&](auto slabs) {
+        constexpr int S = decltype(slabs)::value;
+        auto pick = [&](auto zero) -> int {
+            using T = decltype(zero);
+            if (widest <= 64) return launch(ns_short_conv_kernel<T, 2, S>);
+            return widest <= 128 ? launch(ns_short_conv_kernel<T, 4, S>) : launch(ns_short_conv_kernel<T, 16, S>);
+        };
+        return out_dtype == NS_F32 ? pick(float(0)) : pick(uint16_t(0));
+    });
 }
 
 extern "C" int ns_delta_recurrent(ns_device_t h, uint64_t q, int q_ld, uint64_t k, int k_ld, uint64_t v, int v_ld, uint64_t a_src, int a_splits, int a_ld,

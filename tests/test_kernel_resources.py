@@ -28,7 +28,7 @@ def report():
 @pytest.mark.parametrize("kernel,most_registers,most_spilled", [
     ("ns_lightning_chunk_kernel", 255, 32),
     ("ns_glu_rows_kernel", 48, 0), ("ns_copy_cols_kernel", 32, 0), ("ns_rms_rows_kernel", 40, 0), ("ns_rms_post_rows_kernel", 40, 0),
-    ("ns_window_append_kernel", 48, 40),
+    ("ns_window_append_kernel", 48, 40), ("ns_short_conv_kernel", 72, 20), ("ns_short_conv_slide_kernel", 168, 32),
 ])
 def test_kernels_of_many_rows_stay_small(report, kernel, most_registers, most_spilled):
     builds = {n: v for n, v in report.items() if re.search(r"\d" + kernel + r"(I|E|v)", n)}

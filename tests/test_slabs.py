@@ -93,3 +93,23 @@ def test_window_append(dev, H, G, dim, vdim, steps, splits):
             return q, gate, kr, vr
 
         same(dev, append, source, total, splits)
+
+
+@pytest.mark.parametrize("splits", SPLITS)
+@pytest.mark.parametrize("heads,hd,taps", [(3, 32, 4), (5, 64, 4), (4, 128, 4), (2, 128, 7), (2, 60, 6), (2, 256, 3), (1, 500, 4), (2, 33, 10)])
+@pytest.mark.parametrize("batch,steps", [(2, 1), (70, 2), (2, 40)])
+def test_short_convolution(dev, heads, hd, taps, batch, steps, splits):
+    channels = heads * hd
+    source, total = slabs_and_sum(dev, batch * steps, channels + 4, splits)
+    w, before = (rng_for(4, channels, k).standard_normal(n).astype(np.float32) for k, n in enumerate((channels * taps, batch * taps * channels)))
+    w, slots, pos = dev.from_numpy(w), dev.from_numpy(np.arange(batch, dtype=np.int32)), dev.from_numpy(np.full(batch, 9, np.int32))
+
+    def conv(src, n):
+        hist, out = dev.from_numpy(before), dev.zeros(batch * steps * channels)
+        fields = (C.c_int64 * 9)(4, heads, hd, taps, 1, w.ptr, hist.ptr, out.ptr, channels)
+        N.call("ns_short_conv", dev.handle, u(src.ptr), n, N.NS_F32, channels + 4, 1, fields, (C.c_float * 1)(0.25), i64(taps * channels), u(slots.ptr), u(pos.ptr), batch,
+               steps, N.NS_F32)
+        dev.synchronize()
+        return out, hist
+
+    same(dev, conv, source, total, splits)

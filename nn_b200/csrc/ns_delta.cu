@@ -229,9 +229,10 @@ struct DeltaArgs {
 
 NS_DEVINL float delta_decay(float a, float dt_bias, float rate) { return expf(-rate * ns_softplus(a + dt_bias)); }
 
+// A recurrence is built three ways: slabs in turn, slabs together as the registers come, and slabs together held to CTAS CTAs an SM (0: as they come).
 // 8 warps; warp w holds state rows [w * RPW, (w + 1) * RPW), each lane V neighbouring columns of them, in registers.
-template <int RPW, int V, bool CHANNEL>
-__global__ void __launch_bounds__(256) ns_delta_recurrent_kernel(const DeltaArgs a)
+template <int RPW, int V, bool CHANNEL, int SLABS, int CTAS>
+__global__ void __launch_bounds__(256, CTAS) ns_delta_recurrent_kernel(const DeltaArgs a)
 {
     constexpr int DMAX = RPW * 8, VT = 32 * V, DI = (DMAX + 255) / 256;
     __shared__ float sq[3][DMAX], sk[3][DMAX], sg[3][CHANNEL ? DMAX : 1], sv[3][VT], sbeta[3];
@@ -283,13 +284,13 @@ __global__ void __launch_bounds__(256) ns_delta_recurrent_kernel(const DeltaArgs
             if (c < dim) {
                 pq[j] = a.q[row * a.q_ld + kv * dim + c];
                 pk[j] = a.k[row * a.k_ld + kv * dim + c];
-                if (CHANNEL) pg[j] = ns_source_at(a.a, row * a.a.ld + a.a_col + head * dim + c);
+                if (CHANNEL) pg[j] = ns_source_at<SLABS>(a.a, row * a.a.ld + a.a_col + head * dim + c);
             }
         }
         if (tid < VT) pv = v0 + tid < vdim ? a.v[row * a.v_ld + head * vdim + v0 + tid] : 0.0f;
         if (tid == 0) {
-            pb = ns_source_at(a.b, row * a.b.ld + a.b_col + head);
-            if (!CHANNEL) pg[0] = ns_source_at(a.a, row * a.a.ld + a.a_col + head);
+            pb = ns_source_at<SLABS>(a.b, row * a.b.ld + a.b_col + head);
+            if (!CHANNEL) pg[0] = ns_source_at<SLABS>(a.a, row * a.a.ld + a.a_col + head);
         }
     };
     auto put = [&](int s) {
@@ -460,22 +461,40 @@ __global__ void __launch_bounds__(256) ns_gated_norm_row_kernel(const float* __r
     for (int c = n + threadIdx.x; c < y_ld; c += 256) ns_store(y + row * y_ld + c, 0.0f);
 }
 
-template <int RPW, int V>
-int launch_recurrent(NsDevice* d, const DeltaArgs& a, int batch, bool channel)
+// Many CTAs need warps in flight: slabs in turn where there are two at most, else together in as few registers as that way takes.  Few CTAs
+// need the shortest chain, and have it in the build that holds the most (V = 1: no gain).  16 x 4 values a thread and one decay leave no room
+// for slabs under two CTAs an SM; heads of more than 128 keys hold one an SM either way.  In turn, together, held (us), one decay a head,
+// 16 heads: 64 sequences' step, 4 slabs, 32 x 128 12.3, 13.4, 9.6, 64 x 64 12.6, 13.1, 9.9, 128 x 128 25.4, 29.7, 25.3; one slab of 128 x 128
+// 21.2, 27.3; 7 sequences, 8 slabs, 128 x 128 6.1, 5.1, 5.5; 200 tokens of one, 8 heads of 256 x 256 378, 335.
+template <int RPW, int V, bool CHANNEL>
+int launch_recurrent(NsDevice* d, const DeltaArgs& a, int batch)
 {
+    constexpr int HELD = RPW == 4 ? 4 : (RPW == 8 ? (V == 1 && !CHANNEL ? 4 : 3) : (RPW == 16 ? (CHANNEL || V == 1 ? 2 : (V == 2 ? 3 : 0)) : 0));
     const dim3 grid((unsigned)a.heads, (unsigned)batch, (unsigned)((a.vdim + 32 * V - 1) / (32 * V)));
-    auto k = channel ? ns_delta_recurrent_kernel<RPW, V, true> : ns_delta_recurrent_kernel<RPW, V, false>;
-    NS_CUDA(ns_launch_plain(k, grid, dim3(256), 0, d->stream, a));
-    return NS_OK;
+    const int64_t ctas = (int64_t)grid.x * grid.y * grid.z;
+    const bool slabs = a.a.splits > 2 || a.b.splits > 2, big = RPW == 16 && V == 4 && !CHANNEL;
+    auto go = [&](auto k) -> int {
+        NS_CUDA(ns_launch_plain(k, grid, dim3(256), 0, d->stream, a));
+        return NS_OK;
+    };
+    if (big ? slabs && ctas <= d->sm_count : V > 1 && (RPW == 32 || ctas <= 2 * d->sm_count)) return go(ns_delta_recurrent_kernel<RPW, V, CHANNEL, NS_TOGETHER, 0>);
+    if (slabs && !big) return go(ns_delta_recurrent_kernel<RPW, V, CHANNEL, NS_TOGETHER, HELD>);
+    return go(ns_delta_recurrent_kernel<RPW, V, CHANNEL, NS_IN_TURN, 0>);
+}
+
+template <int V, bool CHANNEL>
+int launch_recurrent_rows(NsDevice* d, const DeltaArgs& a, int batch)
+{
+    if (a.dim <= 32) return launch_recurrent<4, V, CHANNEL>(d, a, batch);
+    if (a.dim <= 64) return launch_recurrent<8, V, CHANNEL>(d, a, batch);
+    if (a.dim <= 128) return launch_recurrent<16, V, CHANNEL>(d, a, batch);
+    return launch_recurrent<32, V, CHANNEL>(d, a, batch);
 }
 
 template <int V>
-int launch_recurrent_rows(NsDevice* d, const DeltaArgs& a, int batch, bool channel)
+int launch_recurrent_of(NsDevice* d, const DeltaArgs& a, int batch, bool channel)
 {
-    if (a.dim <= 32) return launch_recurrent<4, V>(d, a, batch, channel);
-    if (a.dim <= 64) return launch_recurrent<8, V>(d, a, batch, channel);
-    if (a.dim <= 128) return launch_recurrent<16, V>(d, a, batch, channel);
-    return launch_recurrent<32, V>(d, a, batch, channel);
+    return channel ? launch_recurrent_rows<V, true>(d, a, batch) : launch_recurrent_rows<V, false>(d, a, batch);
 }
 
 }  // namespace
@@ -602,9 +621,9 @@ extern "C" int ns_delta_recurrent(ns_device_t h, uint64_t q, int q_ld, uint64_t 
     a.slots = reinterpret_cast<const int32_t*>(slots);
     a.heads = heads; a.kv_heads = kv_heads; a.dim = dim; a.vdim = vdim; a.steps = steps;
     a.o = reinterpret_cast<float*>(o); a.o_ld = o_ld;
-    if (vdim <= 32) return launch_recurrent_rows<1>(d, a, batch, per_channel != 0);
-    if (vdim <= 64) return launch_recurrent_rows<2>(d, a, batch, per_channel != 0);
-    return launch_recurrent_rows<4>(d, a, batch, per_channel != 0);
+    if (vdim <= 32) return launch_recurrent_of<1>(d, a, batch, per_channel != 0);
+    if (vdim <= 64) return launch_recurrent_of<2>(d, a, batch, per_channel != 0);
+    return launch_recurrent_of<4>(d, a, batch, per_channel != 0);
 }
 
 extern "C" int ns_gated_norm(ns_device_t h, uint64_t o, int o_ld, uint64_t gate, int splits, int gate_dtype, int gate_ld, int gate_col, int act, uint64_t w,

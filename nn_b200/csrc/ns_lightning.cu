@@ -36,8 +36,9 @@ struct LightningArgs {
 // ---------------------------------------------------------------------------------------------
 // token by token: 8 warps; warp w holds state rows [w * RPW, (w + 1) * RPW), each lane V neighbouring columns of them
 // ---------------------------------------------------------------------------------------------
-template <int RPW, int V>
-__global__ void __launch_bounds__(256) ns_lightning_recurrent_kernel(const LightningArgs a)
+// Built three ways: slabs in turn, slabs together as the registers come, and slabs together held to CTAS CTAs an SM (0: as they come).
+template <int RPW, int V, int SLABS, int CTAS>
+__global__ void __launch_bounds__(256, CTAS) ns_lightning_recurrent_kernel(const LightningArgs a)
 {
     constexpr int DMAX = RPW * 8, VT = 32 * V;
     __shared__ float sq[2][DMAX], sk[2][DMAX], sv[2][VT], red[2][8][VT];
@@ -55,10 +56,10 @@ __global__ void __launch_bounds__(256) ns_lightning_recurrent_kernel(const Light
     auto fetch = [&](int t) {
         const int64_t at = ((int64_t)b * a.steps + t) * a.src.ld;
         if (tid < dim) {
-            pq = ns_source_at(a.src, at + a.q_col + head * dim + tid);
-            pk = ns_source_at(a.src, at + a.k_col + head * dim + tid);
+            pq = ns_source_at<SLABS>(a.src, at + a.q_col + head * dim + tid);
+            pk = ns_source_at<SLABS>(a.src, at + a.k_col + head * dim + tid);
         }
-        if (tid < VT && v0 + tid < vdim) pv = ns_source_at(a.src, at + a.v_col + head * vdim + v0 + tid);
+        if (tid < VT && v0 + tid < vdim) pv = ns_source_at<SLABS>(a.src, at + a.v_col + head * vdim + v0 + tid);
     };
     auto put = [&](int s) {
         if (tid < DMAX) {
@@ -479,12 +480,24 @@ __global__ void __launch_bounds__(256) ns_lightning_carry_kernel(const Lightning
     *S = x;
 }
 
+// Many CTAs need warps in flight: slabs in turn where there are two at most, else together in as few registers as that way takes (8 x 4 values a
+// thread have no room for that).  Few CTAs need the shortest chain, and have it in the build that holds the most (V = 1: no gain).  In turn,
+// together, held (us), 16 heads: 64 sequences' step, 4 slabs, 64 x 64 9.4, 12.6, 7.5, 64 x 128 12.3, 15.1, 14.3, 128 x 128 25.5, 21.4, 21.5;
+// one slab of 64 x 64 6.3, 10.2; 7 sequences, 8 slabs, 64 x 128 5.1, 3.8; 200 tokens of one, 64 x 64 185, 160; 8 heads of 256 x 32, 64
+// sequences of 4 slabs 11.7, 14.8, 10.2.
 template <int RPW, int V>
 int launch_recurrent(NsDevice* d, const LightningArgs& a, int batch)
 {
+    constexpr int HELD = RPW == 16 || (RPW == 32 && V == 1) ? 2 : (RPW == 4 || (RPW == 8 && V < 4) ? 4 : 0);
     const dim3 grid((unsigned)a.heads, (unsigned)batch, (unsigned)((a.vdim + 32 * V - 1) / (32 * V)));
-    NS_CUDA(ns_launch_plain(ns_lightning_recurrent_kernel<RPW, V>, grid, dim3(256), 0, d->stream, a));
-    return NS_OK;
+    const int64_t ctas = (int64_t)grid.x * grid.y * grid.z;
+    auto go = [&](auto k) -> int {
+        NS_CUDA(ns_launch_plain(k, grid, dim3(256), 0, d->stream, a));
+        return NS_OK;
+    };
+    if (V > 1 && (RPW == 32 || ctas <= 2 * d->sm_count)) return go(ns_lightning_recurrent_kernel<RPW, V, NS_TOGETHER, 0>);
+    if (a.src.splits > 2 && HELD != 0) return go(ns_lightning_recurrent_kernel<RPW, V, NS_TOGETHER, HELD>);
+    return go(ns_lightning_recurrent_kernel<RPW, V, NS_IN_TURN, 0>);
 }
 template <int V>
 int launch_recurrent_rows(NsDevice* d, const LightningArgs& a, int batch)

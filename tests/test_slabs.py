@@ -113,3 +113,50 @@ def test_short_convolution(dev, heads, hd, taps, batch, steps, splits):
         return out, hist
 
     same(dev, conv, source, total, splits)
+
+
+@pytest.mark.parametrize("splits", SPLITS)
+@pytest.mark.parametrize("H,dim,vdim", [(3, 20, 28), (2, 60, 64), (2, 64, 128), (2, 128, 40), (4, 96, 130), (2, 200, 72)])
+@pytest.mark.parametrize("batch,steps", [(2, 3), (170, 1)])
+def test_linear_attention(dev, H, dim, vdim, batch, steps, splits):
+    cols = H * (2 * dim + vdim)
+    source, total = slabs_and_sum(dev, batch * steps, (cols + 7) // 8 * 8, splits)
+    decay = np.linspace(0.5, 1.0, H).astype(np.float32)
+    dec, log2, slots = dev.from_numpy(decay), dev.from_numpy(np.log2(decay)), dev.from_numpy(np.arange(batch, dtype=np.int32))
+    before = rng_for(5, H, dim, vdim, batch).standard_normal(batch * H * dim * vdim).astype(np.float32)
+    for name, extra in (("ns_lightning_recurrent", ()), ("ns_lightning_chunked", (0,))):
+        if name == "ns_lightning_chunked" and dim > 128:
+            continue
+
+        def run(src, n):
+            state, o = dev.from_numpy(before), dev.zeros(batch * steps * H * vdim)
+            N.call(name, dev.handle, u(src.ptr), n, N.NS_F32, (cols + 7) // 8 * 8, 0, H * dim, 2 * H * dim, u(dec.ptr), u(log2.ptr), u(state.ptr), i64(H * dim * vdim),
+                   u(slots.ptr), batch, steps, H, dim, vdim, u(o.ptr), H * vdim, *extra)
+            return o, state
+
+        same(dev, run, source, total, splits)
+
+
+@pytest.mark.parametrize("splits", SPLITS)
+@pytest.mark.parametrize("H,kv,dim,vdim", [(4, 2, 20, 28), (2, 1, 64, 128), (3, 3, 100, 130), (2, 2, 128, 64), (2, 2, 200, 96)])
+@pytest.mark.parametrize("batch,steps", [(2, 3), (170, 1)])
+@pytest.mark.parametrize("channelwise", [0, 1])
+def test_delta_rule(dev, H, kv, dim, vdim, batch, steps, channelwise, splits):
+    rows, ac = batch * steps, H * dim if channelwise else H
+    ld = (ac + H + 7) // 8 * 8
+    source, total = slabs_and_sum(dev, rows, ld, splits)
+    rng = rng_for(6, H, dim, vdim, rows)
+    q, k, v, a_log, dt, before = (rng.standard_normal(s).astype(np.float32) for s in ((rows, kv, dim), (rows, kv, dim), (rows, H * vdim), H, ac, batch * H * dim * vdim))
+    q, k, v, a_log, dt = (dev.from_numpy(a) for a in (q / np.float32(dim ** 0.5), k / np.linalg.norm(k, axis=-1, keepdims=True), v, a_log, dt))
+    slots = dev.from_numpy(np.arange(batch, dtype=np.int32))
+    for name in ("ns_delta_recurrent", "ns_delta_chunked"):
+        if name == "ns_delta_chunked" and dim > 128:
+            continue
+
+        def run(src, n):
+            state, o = dev.from_numpy(before), dev.zeros(rows * H * vdim)
+            N.call(name, dev.handle, u(q.ptr), kv * dim, u(k.ptr), kv * dim, u(v.ptr), H * vdim, u(src.ptr), n, ld, 0, u(src.ptr), n, ld, ac, u(a_log.ptr), u(dt.ptr), channelwise,
+                   u(state.ptr), i64(H * dim * vdim), u(slots.ptr), batch, steps, H, kv, dim, vdim, u(o.ptr), H * vdim)
+            return o, state
+
+        same(dev, run, source, total, splits)

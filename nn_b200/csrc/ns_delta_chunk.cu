@@ -182,8 +182,8 @@ __global__ void __launch_bounds__(256, 1) ns_delta_chunk_kernel(const ChunkArgs 
                 }
             }
         };
-        // ------------------------------------------------------------ step sizes, running decays
-        if (tid < CH) sBeta[tid] = tid < n ? ns_sigmoid(ns_source_at(a.b, (row0 + tid) * a.b.ld + a.b_col + head)) : 0.0f;
+        // ------------------------------------------------------------ step sizes, running decays (slabs in turn: together they spilled)
+        if (tid < CH) sBeta[tid] = tid < n ? ns_sigmoid(ns_source_at<NS_IN_TURN>(a.b, (row0 + tid) * a.b.ld + a.b_col + head)) : 0.0f;
         if (CHANNEL) {
             const int c = (tid % QUADS) * 4;
             const float4 dt = row4(a.dt_bias + (int64_t)head * dim, c, dim);
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(256, 1) ns_delta_chunk_kernel(const ChunkArgs 
                 float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (t < n && c < dim) {
                     const int64_t at = (row0 + t) * a.a.ld + a.a_col + head * dim + c;
-                    x = ns_source_at4(a.a, at);
+                    x = ns_source_at4<NS_IN_TURN>(a.a, at);
                     x = make_float4(fmaxf(-rate2 * softplus(x.x + dt.x), WEAKEST), fmaxf(-rate2 * softplus(x.y + dt.y), WEAKEST),
                                     fmaxf(-rate2 * softplus(x.z + dt.z), WEAKEST), fmaxf(-rate2 * softplus(x.w + dt.w), WEAKEST));
                 }
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(256, 1) ns_delta_chunk_kernel(const ChunkArgs 
 #pragma unroll
             for (int i = 0; i < 2; i++) {
                 const int t = 2 * lane + i;
-                x[i] = t < n ? fmaxf(-rate2 * softplus(ns_source_at(a.a, (row0 + t) * a.a.ld + a.a_col + head) + dt), WEAKEST) : 0.0f;
+                x[i] = t < n ? fmaxf(-rate2 * softplus(ns_source_at<NS_IN_TURN>(a.a, (row0 + t) * a.a.ld + a.a_col + head) + dt), WEAKEST) : 0.0f;
             }
             float s = x[0] + x[1];
 #pragma unroll

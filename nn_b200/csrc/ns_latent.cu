@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(256) ns_latent_append_kernel(const LatentAppen
         }
     } else {
         for (int c = tid; c < n; c += 256) {
-            x[c] = ns_source_at(a.src, base + c);
+            x[c] = ns_source_at<SLABS>(a.src, base + c);
             sum(c, x[c]);
         }
     }
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(256) ns_rotate_heads_kernel(const RotateArgs a
     for (int e = threadIdx.x; e < n; e += blockDim.x) {
         const int head = e / w, c = e - head * w;
         const int64_t at = (int64_t)row * a.src.ld + e;
-        const float x = ns_source_at(a.src, at);
+        const float x = ns_source_at<SLABS>(a.src, at);
         if (c < a.dim) {
             ns_store(reinterpret_cast<TP*>(a.plain) + (int64_t)row * a.plain_ld + (int64_t)head * a.plain_head + c, x);
         } else {
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(256) ns_rotate_heads_kernel(const RotateArgs a
             float y = x;
             if (r < a.rot_dims) {
                 const float2 t = cs[r >> 1];
-                const float other = ns_source_at(a.src, (r & 1) ? at - 1 : at + 1);
+                const float other = ns_source_at<SLABS>(a.src, (r & 1) ? at - 1 : at + 1);
                 y = (r & 1) ? fmaf(x, t.x, other * t.y) : fmaf(x, t.x, -other * t.y);
             }
             ns_store(reinterpret_cast<TR*>(a.rot) + (int64_t)row * a.rot_ld + (int64_t)head * a.rot_head + r, y);
@@ -354,10 +354,15 @@ extern "C" int ns_latent_append(ns_device_t h, uint64_t src, int splits, int src
     const int n = q_rank + kv_rank + rot_dim;
     NS_REQUIRE(n <= 12000, NS_ERR_ARGUMENT, "ns_latent_append: rows of %d values do not fit shared memory", n);
     const bool vec = ((q_rank | kv_rank | rot_dim | src_ld | cq_ld | ring_ld) & 3) == 0 && (ring_slot_stride & 3) == 0 && ((src | q_norm | kv_norm | cq | ring) & 15) == 0;
-    auto k = dtype == NS_F32 ? (!vec ? ns_latent_append_kernel<float, false, NS_TOGETHER> : splits > 1 ? ns_latent_append_kernel<float, true, NS_TOGETHER> : ns_latent_append_kernel<float, true, NS_ONE_SLAB>)
-                             : (!vec ? ns_latent_append_kernel<uint16_t, false, NS_TOGETHER> : splits > 1 ? ns_latent_append_kernel<uint16_t, true, NS_TOGETHER> : ns_latent_append_kernel<uint16_t, true, NS_ONE_SLAB>);
-    NS_CUDA(ns_launch_plain(k, dim3((unsigned)(batch * steps)), dim3(256), (size_t)((n + 3) & ~3) * 4, d->stream, a));
-    return NS_OK;
+    auto go = [&](auto k) -> int {
+        NS_CUDA(ns_launch_plain(k, dim3((unsigned)(batch * steps)), dim3(256), (size_t)((n + 3) & ~3) * 4, d->stream, a));
+        return NS_OK;
+    };
+    return ns_pick_slabs<NS_ONE_SLAB>(splits > 1, [&](auto slabs) {
+        constexpr int S = decltype(slabs)::value;
+        if (dtype == NS_F32) return vec ? go(ns_latent_append_kernel<float, true, S>) : go(ns_latent_append_kernel<float, false, S>);
+        return vec ? go(ns_latent_append_kernel<uint16_t, true, S>) : go(ns_latent_append_kernel<uint16_t, false, S>);
+    });
 }
 
 extern "C" int ns_rotate_heads(ns_device_t h, uint64_t src, int splits, int src_dtype, int src_ld, int heads, int dim, int rot_dim, int rot_dims, uint64_t freq,
@@ -382,10 +387,13 @@ extern "C" int ns_rotate_heads(ns_device_t h, uint64_t src, int splits, int src_
         NS_CUDA(ns_launch_plain(kern, dim3((unsigned)(batch * steps)), dim3(256), (size_t)(rot_dims / 2 + 1) * sizeof(float2), d->stream, a));
         return NS_OK;
     };
-    if (plain_dtype == NS_F32 && rot_dtype == NS_F32) return !vec ? go(ns_rotate_heads_kernel<float, float, false, NS_TOGETHER>) : splits > 1 ? go(ns_rotate_heads_kernel<float, float, true, NS_TOGETHER>) : go(ns_rotate_heads_kernel<float, float, true, NS_ONE_SLAB>);
-    if (plain_dtype == NS_BF16 && rot_dtype == NS_BF16)
-        return !vec ? go(ns_rotate_heads_kernel<uint16_t, uint16_t, false, NS_TOGETHER>) : splits > 1 ? go(ns_rotate_heads_kernel<uint16_t, uint16_t, true, NS_TOGETHER>) : go(ns_rotate_heads_kernel<uint16_t, uint16_t, true, NS_ONE_SLAB>);
-    return ns_fail(NS_ERR_ARGUMENT, "ns_rotate_heads: both outputs have one type");
+    // value by value, 8000 rows of 16 heads of 127 + 30: 77 us in the build for many slabs, 55 in its own
+    if (plain_dtype != rot_dtype) return ns_fail(NS_ERR_ARGUMENT, "ns_rotate_heads: both outputs have one type");
+    return ns_pick_slabs<NS_ONE_SLAB>(splits > 1, [&](auto slabs) {
+        constexpr int S = decltype(slabs)::value;
+        if (plain_dtype == NS_F32) return vec ? go(ns_rotate_heads_kernel<float, float, true, S>) : go(ns_rotate_heads_kernel<float, float, false, S>);
+        return vec ? go(ns_rotate_heads_kernel<uint16_t, uint16_t, true, S>) : go(ns_rotate_heads_kernel<uint16_t, uint16_t, false, S>);
+    });
 }
 
 extern "C" int ns_head_matmul(ns_device_t h, int x_dtype, uint64_t x, int64_t x_ld, int x_head, int w_dtype, uint64_t w, int64_t w_head, int64_t w_k, int64_t w_n,

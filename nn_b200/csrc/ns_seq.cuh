@@ -45,7 +45,7 @@ static inline int ns_pick_slabs(bool together, F f)
 }
 
 // the value at element `idx` (row * ld + column)
-template <int SLABS = NS_TOGETHER>
+template <int SLABS>
 NS_DEVINL float ns_source_at(const NsSource& s, int64_t idx)
 {
     if (s.dtype == NS_BF16) return ns_bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(s.ptr)[idx]);
@@ -68,7 +68,7 @@ NS_DEVINL float ns_source_at(const NsSource& s, int64_t idx)
 }
 NS_DEVINL float4 ns_add4(float4 v, float4 t) { return make_float4(__fadd_rn(v.x, t.x), __fadd_rn(v.y, t.y), __fadd_rn(v.z, t.z), __fadd_rn(v.w, t.w)); }
 // four consecutive values; idx and ld are multiples of 4 and ptr is 16-byte aligned
-template <int SLABS = NS_TOGETHER>
+template <int SLABS>
 NS_DEVINL float4 ns_source_at4(const NsSource& s, int64_t idx)
 {
     if (s.dtype == NS_BF16) {

@@ -29,7 +29,7 @@ def report():
     ("ns_lightning_chunk_kernel", 255, 32),
     ("ns_glu_rows_kernel", 48, 0), ("ns_copy_cols_kernel", 32, 0), ("ns_rms_rows_kernel", 40, 0), ("ns_rms_post_rows_kernel", 40, 0),
     ("ns_window_append_kernel", 48, 40), ("ns_short_conv_kernel", 72, 20), ("ns_short_conv_slide_kernel", 168, 32),
-    ("ns_delta_chunk_kernel", 254, 0),
+    ("ns_rotate_heads_kernel", 32, 0), ("ns_latent_append_kernel", 40, 0), ("ns_gated_norm_kernel", 48, 0), ("ns_delta_chunk_kernel", 254, 0),
     ("ns_delta_recurrent_kernelILi16E", 128, 0), ("ns_lightning_recurrent_kernelILi8E", 64, 24),
 ])
 def test_kernels_of_many_rows_stay_small(report, kernel, most_registers, most_spilled):

@@ -160,3 +160,45 @@ def test_delta_rule(dev, H, kv, dim, vdim, batch, steps, channelwise, splits):
             return o, state
 
         same(dev, run, source, total, splits)
+
+
+@pytest.mark.parametrize("splits", SPLITS)
+@pytest.mark.parametrize("rows,heads,vdim", [(3, 2, 64), (3, 2, 61), (300, 16, 128), (5, 1, 1028), (2, 1, 4100), (2, 1, 601)])
+def test_gated_norm(dev, rows, heads, vdim, splits):
+    n = heads * vdim
+    ld = (n + 7) // 8 * 8
+    source, total = slabs_and_sum(dev, rows, ld, splits)
+    o, w = (dev.from_numpy(rng_for(7, k, n).standard_normal(k).astype(np.float32)) for k in (rows * ld, vdim))
+    for out in (N.NS_F32, N.NS_BF16):
+        def norm(src, k):
+            y = dev.zeros(rows * ld, out)
+            N.call("ns_gated_norm", dev.handle, u(o.ptr), ld, u(src.ptr), k, N.NS_F32, ld, 0, N.ACT_SILU, u(w.ptr), fl(1e-4), i64(rows), heads, vdim, out, u(y.ptr), ld)
+            return (y,)
+
+        same(dev, norm, source, total, splits)
+
+
+@pytest.mark.parametrize("splits", SPLITS)
+@pytest.mark.parametrize("q_rank,kv_rank,rot", [(64, 32, 16), (61, 31, 14), (1024, 512, 64)])
+def test_latent_rows(dev, q_rank, kv_rank, rot, splits):
+    batch, steps, ring, n = 2, 5, 16, q_rank + kv_rank + rot
+    ld, q_ld, r_ld, heads = (n + 7) // 8 * 8, (q_rank + 7) // 8 * 8, (kv_rank + rot + 7) // 8 * 8, 2
+    source, total = slabs_and_sum(dev, batch * steps, ld, splits)
+    wq, wk, freq = (dev.from_numpy(rng_for(8, k).standard_normal(k).astype(np.float32)) for k in (q_rank, kv_rank, rot // 2))
+    slots, pos = dev.from_numpy(np.array([1, 0], np.int32)), dev.from_numpy(np.array([3, 14], np.int32))
+    for dtype in (N.NS_F32, N.NS_BF16):
+        def append(src, k):
+            cq, rows = dev.zeros(batch * steps * q_ld, dtype), dev.zeros(2 * ring * r_ld, dtype)
+            N.call("ns_latent_append", dev.handle, u(src.ptr), k, N.NS_F32, ld, q_rank, kv_rank, rot, rot, u(wq.ptr), u(wk.ptr), fl(1e-4), u(freq.ptr), u(slots.ptr), u(pos.ptr),
+                   batch, steps, dtype, u(cq.ptr), q_ld, u(rows.ptr), i64(ring * r_ld), ring, r_ld)
+            return cq, rows
+
+        def rotate(src, k):
+            dim = n // heads - rot
+            plain, turned = dev.zeros(batch * steps * heads * dim, dtype), dev.zeros(batch * steps * heads * rot, dtype)
+            N.call("ns_rotate_heads", dev.handle, u(src.ptr), k, N.NS_F32, ld, heads, dim, rot, rot, u(freq.ptr), u(slots.ptr), u(pos.ptr), batch, steps, dtype, u(plain.ptr),
+                   i64(heads * dim), dim, dtype, u(turned.ptr), i64(heads * rot), rot)
+            return plain, turned
+
+        for run in (append, rotate):
+            same(dev, run, source, total, splits)

@@ -361,7 +361,8 @@ extern "C" int ns_f32_embed_positions(ns_device_t h, uint64_t ids, uint64_t tabl
     const int64_t n = (int64_t)batch * steps * dim;
     if (n == 0) return NS_OK;
     const int64_t blocks = (n + 255) / 256, cap = (int64_t)d->sm_count * 16;
-    NS_CUDA(ns_launch_pdl(ns_f32_embed_positions_kernel, dim3((unsigned)(blocks < cap ? blocks : cap)), dim3(256), 0, d->stream, reinterpret_cast<const float*>(ids),
+    // nothing to do before its inputs are there: no programmatic start (it lets the first product start early all the same)
+    NS_CUDA(ns_launch_plain(ns_f32_embed_positions_kernel, dim3((unsigned)(blocks < cap ? blocks : cap)), dim3(256), 0, d->stream, reinterpret_cast<const float*>(ids),
                           reinterpret_cast<const float*>(table), reinterpret_cast<const float*>(positions), reinterpret_cast<const float*>(position),
                           reinterpret_cast<float*>(x), batch * steps, steps, dim, vocabulary, capacity));
     return NS_OK;

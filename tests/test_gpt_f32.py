@@ -62,6 +62,23 @@ def test_batched_decoding_and_graph_replay(dev, orc):
         assert orc.close(ref.logit_trace[s], trace_b[s], 1e-4)
 
 
+@pytest.mark.parametrize("batch,steps,position", [(1, 1, 0), (3, 1, 6), (2, 4, 4), (2, 3, 9)])
+def test_step_embedding_has_the_operators_bits(dev, orc, batch, steps, position):
+    """Ids and positions past their tables, fractions and negative ids are taken as Gather takes them."""
+    be, D, V, cap, n = NsB200Backend(dev), 20, 11, 7, batch * steps
+    up = lambda a: dev.from_numpy(np.ascontiguousarray(a, dtype=np.float32))
+    table, places = up(orc.normal((V, D), 95)), up(orc.normal((cap, D), 96))
+    ids = up(np.resize([3.0, 10.0, 11.0, 1e9, -2.0, 0.0, 4.7, 9.0], n))
+    where, pos = up(np.resize(position + np.arange(steps), n)), up([position])
+    x, t, e = dev.empty(n * D), dev.empty(n * D), dev.empty(n * D)
+    N.call("ns_f32_embed_positions", dev.handle, ids.ptr, table.ptr, places.ptr, pos.ptr, x.ptr, batch, steps, D, V, cap)
+    be.Gather(table, ids, t, n, D, V)
+    be.Gather(places, where, e, n, D, cap)
+    be.Add(t, e, t, n * D)
+    dev.synchronize()
+    assert np.array_equal(x.download().view(np.uint32), t.download().view(np.uint32))
+
+
 @pytest.mark.parametrize("sinusoid", [False, True])
 def test_baseline_config_1(dev, orc, sinusoid):
     cfg = GptConfig(vocab=96, dim=128, heads=4, layers=4, ff_dim=512, context=128)

@@ -1,5 +1,7 @@
-"""Registers and spills of the kernels that read partial sums, as the compiler reports them (build/*.ptxas).  A kernel that holds the values of many
-slabs where a prompt has one finished matrix loses warps in flight, or spills, and no result shows it."""
+"""What no result shows.  Registers and spills of the kernels that read partial sums, as the compiler reports them (build/*.ptxas): a kernel that holds
+the values of many slabs where a prompt has one finished matrix loses warps in flight, or spills.  And the pointers of kernels that may start
+before the one in front of them has finished."""
+import glob
 import os
 import re
 
@@ -43,3 +45,14 @@ def test_kernels_of_many_rows_stay_small(report, kernel, most_registers, most_sp
         key = re.sub(r"(Li\d+E){%d}E" % ways, "E", name)
         sizes[key] = min(regs, sizes.get(key, 1 << 30))
     assert max(sizes.values()) <= most_registers, sizes
+
+
+def test_programmatic_launches_read_nothing_early():
+    """The compiler may move a load through a const __restrict__ pointer above griddepcontrol.wait, unless the pointer comes out of ns_after_wait."""
+    source = "\n".join(open(f).read() for f in sorted(glob.glob(os.path.join(build.CSRC, "*.cu"))))
+    names = set(re.findall(r"ns_launch_pdl\(\s*(ns_\w+?)(?:<[^(]*>)?,", source))
+    assert "ns_f32_linear_kernel" in names and "ns_f32_attention_step_kernel" in names
+    for name in names:
+        parameters, body = re.search(name + r"\(([^)]*)\)\s*\{(.*?)\n\}", source, re.S).groups()
+        for pointer in re.findall(r"const\s+\w+\*\s*__restrict__\s+(\w+)", parameters):
+            assert re.search(r"\b%s = ns_after_wait\(%s\)" % (pointer, pointer), body), (name, pointer)

@@ -5,8 +5,8 @@
 // one for the output: 215 us a token for four layers of width 128, whose weights are read in a tenth of a microsecond.  Here a product
 // takes the LayerNorm in front of it and the bias, GELU and residual behind it, one kernel does what lies between two
 // products of the attention, and the kernels are launched programmatically: a product has its first weights in shared memory before
-// its input is ready.  Every output is the same chain of operations as in the operators, so the bits are the same.  Measured on
-// that decoder (context 128, one sequence): 128 tokens from a prompt of 32 34.4 -> 15.8 ms, a step on the GPU 215 -> 95 us.
+// its input is ready.  Every output is the same chain of operations as in the operators, so the bits are the same (of finite caches).
+// Measured on that decoder (context 128, one sequence): 128 tokens from a prompt of 32 34.4 -> 15.8 ms, a step on the GPU 215 -> 95 us.
 #include "ns_common.cuh"
 
 namespace {
@@ -25,6 +25,7 @@ struct LinearF32Args {
     const float* residual;   // [m, n] or null
     float* y;
     int m, n, k, gelu;
+    int turned;              // 1: rows of tiles along x, which takes more of them than y does
 };
 
 __device__ __forceinline__ void copy16_async(float* dst, const float* src)
@@ -111,7 +112,7 @@ __global__ void __launch_bounds__(32 * L_WARPS) ns_f32_linear_kernel(const Linea
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* rows_smem = reinterpret_cast<float*>(linear_smem);              // [8 R][k]
     float* ring = rows_smem + (size_t)R * L_WARPS * a.k;                  // [L_STAGES][LK][L_LD]
-    const int col0 = blockIdx.x * LT, row0 = (blockIdx.y * L_WARPS + warp) * R;
+    const int col0 = (int)(a.turned ? blockIdx.y : blockIdx.x) * LT, row0 = ((int)(a.turned ? blockIdx.x : blockIdx.y) * L_WARPS + warp) * R;
     const int slices = (a.k + LK - 1) / LK;
 
     auto load_w = [&](int slice) {
@@ -181,7 +182,8 @@ __global__ void __launch_bounds__(32 * L_WARPS) ns_f32_linear_kernel(const Linea
 // ------------------------------------------------------------------------------------------------
 // One new position per sequence: this (sequence, head)'s key and value into the cache, scores over the positions there are, softmax,
 // weighted values, heads side by side.  One CTA per (sequence, head).  Positions past the current one have weight exp(-1e9 - max) = 0 in
-// the operators and are left out; the sums are those of ns_f32_scale_mask_softmax_kernel's 128 threads in their order.
+// the operators and are left out, which comes to the same wherever the cache is finite; the sums are those of
+// ns_f32_scale_mask_softmax_kernel's 128 threads in their order.
 // ------------------------------------------------------------------------------------------------
 struct AttentionStepF32Args {
     const float* qkv;        // [batch, 3 heads dim]
@@ -296,7 +298,7 @@ __global__ void ns_f32_embed_positions_kernel(const float* __restrict__ ids, con
     }
 
 template <int R>
-static int launch_linear(NsDevice* d, const LinearF32Args& a)
+static int launch_linear(NsDevice* d, LinearF32Args a)
 {
     constexpr int ring = L_STAGES * LK * L_LD * (int)sizeof(float);
     static bool configured[64] = {false};
@@ -304,7 +306,10 @@ static int launch_linear(NsDevice* d, const LinearF32Args& a)
         NS_CUDA(cudaFuncSetAttribute(ns_f32_linear_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, LINEAR_A_BYTES + ring));
         configured[d->ordinal] = true;
     }
-    const dim3 grid((a.n + LT - 1) / LT, (a.m + L_WARPS * R - 1) / (L_WARPS * R));
+    const unsigned across = (unsigned)(((int64_t)a.n + LT - 1) / LT), down = (unsigned)(((int64_t)a.m + L_WARPS * R - 1) / (L_WARPS * R));
+    a.turned = down > 65535;
+    NS_REQUIRE(!a.turned || across <= 65535, NS_ERR_ARGUMENT, "ns_f32_linear: %d x %d is too large", a.m, a.n);
+    const dim3 grid = a.turned ? dim3(down, across) : dim3(across, down);
     NS_CUDA(ns_launch_pdl(ns_f32_linear_kernel<R>, grid, dim3(32 * L_WARPS), (size_t)R * L_WARPS * a.k * 4 + ring, d->stream, a));
     return NS_OK;
 }
@@ -317,7 +322,7 @@ extern "C" int ns_f32_linear(ns_device_t h, uint64_t x, uint64_t gamma, uint64_t
     NS_REQUIRE((gamma == 0) == (beta == 0), NS_ERR_ARGUMENT, "ns_f32_linear: gamma and beta go together");
     NS_REQUIRE(((n | k) & 3) == 0 && ((x | w) & 15) == 0, NS_ERR_ARGUMENT, "ns_f32_linear: n=%d and k=%d must be multiples of 4, x and w on 16 bytes", n, k);
     NS_REQUIRE(k <= LINEAR_A_BYTES / 4 / L_WARPS, NS_ERR_ARGUMENT, "ns_f32_linear: k=%d is more than %d", k, LINEAR_A_BYTES / 4 / L_WARPS);
-    NS_REQUIRE(((int64_t)m + L_WARPS - 1) / L_WARPS <= 65535, NS_ERR_ARGUMENT, "ns_f32_linear: %d rows are more than a step has", m);
+    NS_REQUIRE(m <= (1 << 30), NS_ERR_ARGUMENT, "ns_f32_linear: %d rows are too many", m);
     if (m == 0) return NS_OK;
     LinearF32Args a;
     a.x = reinterpret_cast<const float*>(x); a.gamma = reinterpret_cast<const float*>(gamma); a.beta = reinterpret_cast<const float*>(beta);
@@ -338,6 +343,7 @@ extern "C" int ns_f32_attention_step(ns_device_t h, uint64_t qkv, uint64_t keys,
     NS_REQUIRE((dim & 3) == 0 && ((qkv | keys | values) & 15) == 0, NS_ERR_ARGUMENT, "ns_f32_attention_step: dim=%d must be a multiple of 4, operands on 16 bytes", dim);
     const int64_t smem = ((int64_t)capacity * dim + capacity + dim) * 4;
     NS_REQUIRE(smem <= 200 * 1024, NS_ERR_ARGUMENT, "ns_f32_attention_step: %d positions of %d do not fit shared memory", capacity, dim);
+    NS_REQUIRE((int64_t)batch * heads < ((int64_t)1 << 31), NS_ERR_ARGUMENT, "ns_f32_attention_step: %d sequences of %d heads are too many", batch, heads);
     if (batch == 0) return NS_OK;
     static bool configured[64] = {false};
     if (!configured[d->ordinal]) {

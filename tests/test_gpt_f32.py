@@ -106,7 +106,7 @@ def test_baseline_config_1(dev, orc, sinusoid):
 
 
 # around a warp's rows (1, 2 and 4 of tiles of 8, 16 and 32), a tile's 32 columns, the ring's 64-step slices (8 of them), the longest row of each form
-@pytest.mark.parametrize("m,n,k", [(1, 4, 4), (1, 128, 512), (3, 36, 60), (8, 32, 64), (9, 28, 452), (17, 100, 516), (33, 64, 1024), (17, 32, 1028), (9, 8, 2052), (2, 8, 4096)])
+@pytest.mark.parametrize("m,n,k", [(1, 4, 4), (1, 128, 512), (3, 36, 60), (8, 32, 64), (9, 28, 452), (17, 100, 516), (33, 64, 1024), (17, 32, 1028), (9, 8, 2052), (2, 8, 4096), (2097153, 4, 4)])
 def test_step_linear_has_the_operators_bits(dev, orc, m, n, k):
     be = NsB200Backend(dev)
     up = lambda a: dev.from_numpy(np.ascontiguousarray(a, dtype=np.float32))

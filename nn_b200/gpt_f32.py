@@ -55,6 +55,13 @@ class GptF32:
         self.length = 0
         # sizes the step kernels take: vectors of four floats, an input row of each product and a head's values in shared memory
         self.step_kernels = D % 4 == 0 and FF % 4 == 0 and V % 4 == 0 and dh % 4 == 0 and max(D, FF) <= 4096 and (cap * dh + cap + dh) * 4 <= 200 * 1024
+        # They read the weights once for every 32 rows (vectors of up to 1024), 16 (up to 2048) or 8, the operators once for every 64: of many sequences
+        # the operators are faster where the vectors are long.  Us a step of two layers, kernels against operators, by width / FFN: 512 / 4096, 256
+        # sequences 991, 1119, 1024 3621, 3503; 768 / 3072, 1024 4715, 5028; 1024 / 2048, 1024 4703, 5425; 1024 / 4096, 64 790, 867, 128 1357, 1320;
+        # 2048 / 2048, 96 1507, 1864, 256 3682, 3092; 2048 / 4096, 8 392, 545, 64 1478, 1211.
+        if max(D, FF) > 2048 or D > 1024:
+            most = 512 if D <= 768 else 96 if min(D, FF) <= 1024 or max(D, FF) <= 2048 else 32
+            self.step_kernels = self.step_kernels and batch <= most
         self.graph = None
         self.sampler = None                         # a TokenSampler replaces the greedy choice (CharGpt.cs:283-300)
 

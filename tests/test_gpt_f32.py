@@ -62,6 +62,13 @@ def test_batched_decoding_and_graph_replay(dev, orc):
         assert orc.close(ref.logit_trace[s], trace_b[s], 1e-4)
 
 
+@pytest.mark.parametrize("dim,ff,batch,kernels", [(8, 2048, 600, True), (8, 2052, 512, True), (8, 2052, 513, False), (772, 2052, 96, True), (772, 2052, 97, False),
+                                                  (1028, 8, 96, True), (1028, 8, 97, False), (1028, 2052, 32, True), (1028, 2052, 33, False), (8, 4100, 1, False)])
+def test_step_kernels_are_taken_where_they_are_faster(dev, orc, dim, ff, batch, kernels):
+    cfg = GptConfig(vocab=8, dim=dim, heads=2, layers=1, ff_dim=ff, context=4)
+    assert GptF32(dev, cfg, om.make_weights(cfg, seed=1), batch, max_steps=1).step_kernels == kernels
+
+
 @pytest.mark.parametrize("batch,steps,position", [(1, 1, 0), (3, 1, 6), (2, 4, 4), (2, 3, 9)])
 def test_step_embedding_has_the_operators_bits(dev, orc, batch, steps, position):
     """Ids and positions past their tables, fractions and negative ids are taken as Gather takes them."""

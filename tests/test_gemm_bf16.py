@@ -141,5 +141,6 @@ def test_few_rows(dev, orc, m, n, k):
     b = orc.round_bf16(orc.normal((n, k), 62))
     c = _run(dev, a, b, m, n, k, True, out_dtype=N.NS_F32)[0]
     exp = orc.matmul_bf16(a, b, b_is_nk=True)
-    # sums in another order: K * 2^-23 of the terms' magnitudes (mean |a b| of normal values is 2 / pi, four times that at the most)
-    assert np.max(np.abs(exp - c)) <= k * 2.0 ** -23 * k * 2.0
+    # Sums in another order.  A partial sum is about sqrt(K) large and a rounding 2^-24 of it: K of random sign make K 2^-24, taken five times for the
+    # outliers among the outputs and four times for accumulators that cut off.  2056 terms: 2.5e-3, where one lost term is 0.6 on average.
+    assert np.max(np.abs(exp - c)) <= 20 * k * 2.0 ** -24

@@ -19,12 +19,15 @@ from oracle import model as om
 
 pytestmark = pytest.mark.gpu
 TINY = GptConfig(vocab=11, dim=16, heads=4, layers=2, ff_dim=32, context=12)
+TINY12 = GptConfig(vocab=12, dim=16, heads=4, layers=2, ff_dim=32, context=12)     # a vocabulary the step kernels take
 
 
-def test_cached_decoding_matches_full(dev, orc):
+@pytest.mark.parametrize("TINY", [TINY, TINY12], ids=["operators", "step kernels"])
+def test_cached_decoding_matches_full(dev, orc, TINY):
     w = om.make_weights(TINY, seed=7, std=0.3, sinusoid=True)
     ids = orc.token_ids((1, 10), 70, TINY.vocab).astype(np.int64)
     m = GptF32(dev, TINY, w, 1, max_steps=10)
+    assert m.step_kernels == (TINY.vocab == 12)
     # full forward over 10 positions
     m.prefill(ids)
     dev.synchronize()
@@ -42,7 +45,8 @@ def test_cached_decoding_matches_full(dev, orc):
     assert orc.close(full, np.concatenate(rows), 1e-4)
 
 
-def test_batched_decoding_and_graph_replay(dev, orc):
+@pytest.mark.parametrize("TINY", [TINY, TINY12], ids=["operators", "step kernels"])
+def test_batched_decoding_and_graph_replay(dev, orc, TINY):
     w = om.make_weights(TINY, seed=8, std=0.3, sinusoid=True)
     prompts = orc.token_ids((3, 3), 71, TINY.vocab).astype(np.int64)
     together = GptF32(dev, TINY, w, 3, max_steps=6)
@@ -62,8 +66,26 @@ def test_batched_decoding_and_graph_replay(dev, orc):
         assert orc.close(ref.logit_trace[s], trace_b[s], 1e-4)
 
 
-@pytest.mark.parametrize("dim,ff,batch,kernels", [(8, 2048, 600, True), (8, 2052, 512, True), (8, 2052, 513, False), (772, 2052, 96, True), (772, 2052, 97, False),
-                                                  (1028, 8, 96, True), (1028, 8, 97, False), (1028, 2052, 32, True), (1028, 2052, 33, False), (8, 4100, 1, False)])
+@pytest.mark.parametrize("use_graph", [False, True])
+@pytest.mark.parametrize("batch", [1, 3, 9])
+def test_steps_have_the_operators_bits(dev, orc, batch, use_graph):
+    """The same model with and without the step kernels, across a context reset: tokens, logits and caches."""
+    cfg = GptConfig(vocab=40, dim=48, heads=3, layers=2, ff_dim=100, context=20)
+    w = om.make_weights(cfg, seed=9, std=0.3)
+    prompts = orc.token_ids((batch, 5), 72, cfg.vocab).astype(np.int64)
+    models = [GptF32(dev, cfg, w, batch, max_steps=10) for _ in range(2)]
+    assert models[0].step_kernels
+    models[1].step_kernels = False
+    (tok, resets, trace), (tok_o, resets_o, trace_o) = (m.generate(prompts, 24, use_graph) for m in models)
+    assert resets == resets_o == 1 and np.array_equal(tok, tok_o)
+    for a, b in zip(trace, trace_o):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    for a, b in zip(models[0].keys + models[0].values, models[1].keys + models[1].values):
+        assert np.array_equal(a.download().view(np.uint32), b.download().view(np.uint32))
+
+
+@pytest.mark.parametrize("dim,ff,batch,kernels", [(8, 2048, 600, True), (8, 2052, 512, True), (8, 2052, 513, False), (776, 2052, 96, True), (776, 2052, 97, False),
+                                                  (1032, 8, 96, True), (1032, 8, 97, False), (1032, 2052, 32, True), (1032, 2052, 33, False), (8, 4100, 1, False)])
 def test_step_kernels_are_taken_where_they_are_faster(dev, orc, dim, ff, batch, kernels):
     cfg = GptConfig(vocab=8, dim=dim, heads=2, layers=1, ff_dim=ff, context=4)
     assert GptF32(dev, cfg, om.make_weights(cfg, seed=1), batch, max_steps=1).step_kernels == kernels

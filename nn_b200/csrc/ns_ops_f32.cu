@@ -445,9 +445,17 @@ extern "C" int ns_f32_batched_matmul(ns_device_t h, uint64_t a, uint64_t b, uint
         const float *pa = CF32P(a) + (size_t)b0 * m * k, *pb = CF32P(b) + (size_t)b0 * k * n;
         float* pc = F32P(c) + (size_t)b0 * m * n;
         dim3 grid((n + FT - 1) / FT, (m + FT - 1) / FT, nb);
-        // few 64 x 64 tiles, or tiles that would be half empty: small tiles.  Measured (us, small against large) at n = k = 2048:
-        // 256 rows (128 large tiles) 188 against 227, 300 rows (160) 231 against 277, 400 rows (224) 304 against 280.
-        if (m <= ST || (int64_t)grid.x * grid.y * grid.z * 4 < (int64_t)d->sm_count * 5) {
+        // Few 64 x 64 tiles: small tiles (us, small against large, n = k = 2048: 256 rows, 128 large tiles, 188, 227; 300 rows, 160, 231, 277; 400
+        // rows, 224, 304, 280).  Many of at most 32 rows, half of a large tile or more left empty: small tiles from a number of steps on that
+        // pays for setting up their ring, and grows with the rows that are there; two or three CTAs an SM hide a shorter one, and at most 32
+        // columns leave half of the large tile's width empty too.  1024 products of 128 columns: 1 row, 32 steps 22, 25, B transposed 27, 25,
+        // 48 steps 26, 36 and 34, 37; 16 rows, 48 steps 34, 38 and 41, 38, 64 steps 34, 48 and 38, 49; 32 rows, 64 steps 45, 49 and 49, 50,
+        // 65 steps 56, 53 and 69, 55; 512 of 32 rows, 128 steps 42, 49 and 46, 51.  Of 1000 columns and 16 steps: 1 row 143, 97, 32 rows 270,
+        // 145.  128 products of 1 x 128, 32 steps 4.0, 5.7.  8192 of 32 x 32, 32 steps 76, 115.
+        const int64_t tiles = (int64_t)grid.x * grid.y * grid.z;
+        const int least = !transB && m <= 16 ? (m <= 4 ? 32 : 48) : (m <= 8 ? 48 : (m <= 16 || k == SK ? SK : 2 * SK));
+        const bool shallow = k >= 32 && (n <= ST || (m <= 16 && tiles <= 2 * d->sm_count));
+        if (tiles * 4 < (int64_t)d->sm_count * 5 || (m <= ST && (k >= least || shallow))) {
             grid = dim3((n + ST - 1) / ST, (m + ST - 1) / ST, nb);
             ns_f32_matmul_small_kernel<<<grid, 256, smem, d->stream>>>(pa, pb, pc, m, n, k, transA, transB, beta);
         } else {

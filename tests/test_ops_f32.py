@@ -39,9 +39,12 @@ def test_matmul_reference(dev, orc, m, n, k):
                 assert orc.close(A @ B + beta * c0[0], got[0], 1e-4)
 
 
-# around the small-tile kernel's rows (4 a thread, 32 a tile), columns and k slices (64, six in a ring), and around the line to the large tiles
+# around the small-tile kernel's rows (4 a thread, 32 a tile), columns and k slices (64, six in a ring)
 @pytest.mark.parametrize("batch,m,n,k", [(1, 1, 32, 64), (1, 1, 33, 65), (2, 2, 31, 63), (1, 5, 64, 384), (1, 4, 97, 449), (3, 32, 1, 7), (1, 33, 40, 320), (1, 31, 6000, 30),
-                                         (1, 33, 5888, 33), (1, 33, 5889, 33)])
+                                         (1, 33, 5888, 33), (1, 33, 5889, 33),
+                                         # many products of few rows, around the steps and columns from which they take small tiles
+                                         (200, 1, 128, 47), (200, 8, 128, 48), (200, 9, 128, 48), (200, 9, 200, 31), (130, 16, 128, 32), (200, 16, 130, 64), (200, 17, 100, 65),
+                                         (200, 32, 100, 64), (200, 32, 100, 127), (200, 20, 100, 128), (700, 32, 32, 31), (700, 32, 32, 32), (400, 3, 33, 32)])
 def test_small_products(dev, orc, batch, m, n, k):
     for ta in (False, True):
         for tb in (False, True):
@@ -50,6 +53,24 @@ def test_small_products(dev, orc, batch, m, n, k):
             c0 = orc.normal((batch, m, n), 13 + k)
             got = _mm(dev, a, b, c0, batch, m, n, k, ta, tb, 0.5)
             exp = orc.matmul_f32(a, b, batch, m, n, k, ta, tb, 0.5, c=c0)
+            assert np.array_equal(got.view(np.uint32), exp.reshape(got.shape).view(np.uint32)), (ta, tb)
+
+
+@pytest.mark.parametrize("beta", [0.0, 0.5, 1.0])
+@pytest.mark.parametrize("case", ["last small", "first large", "batch", "rows"])
+def test_products_on_both_sides_of_the_line(dev, orc, case, beta):
+    """The first product with a quarter more 64 x 64 tiles than SMs goes to the large tiles, the one before it does not; batches and odd
+    rows of the large tiles."""
+    line = (5 * dev.sm_count + 3) // 4
+    batch, m, n, k = {"last small": (1, 33, (line - 1) * 64, 33), "first large": (1, 33, (line - 1) * 64 + 1, 33), "batch": ((line + 3) // 4, 65, 67, 19),
+                      "rows": (1, (line - 1) * 64 + 1, 35, 17)}[case]
+    for ta in (False, True):
+        for tb in (False, True):
+            a = orc.normal((batch, k, m) if ta else (batch, m, k), 21 + m % 7)
+            b = orc.normal((batch, n, k) if tb else (batch, k, n), 22 + n % 7)
+            c0 = orc.normal((batch, m, n), 23 + k)
+            got = _mm(dev, a, b, c0, batch, m, n, k, ta, tb, beta)
+            exp = orc.matmul_f32(a, b, batch, m, n, k, ta, tb, beta, c=c0)
             assert np.array_equal(got.view(np.uint32), exp.reshape(got.shape).view(np.uint32)), (ta, tb)
 
 

@@ -25,7 +25,6 @@ struct LinearF32Args {
     const float* residual;   // [m, n] or null
     float* y;
     int m, n, k, gelu;
-    int turned;              // 1: rows of tiles along x, which takes more of them than y does
 };
 
 __device__ __forceinline__ void copy16_async(float* dst, const float* src)
@@ -105,14 +104,15 @@ __device__ __forceinline__ void chains(const float* as, int a_ld, const float* b
 // A tile is 8 R rows of 32 columns: a warp owns R rows (loads them, normalises them, multiplies them), a lane one column.  What bounds it is
 // latency: one trip for the input rows, k dependent multiply-adds (4 cycles each), so the weights run ahead through a ring of
 // 64-step slices (16-byte asynchronous copies; the first 448 steps are under way before the input is ready).
-template <int R>
+// TURNED: rows of tiles along x, which takes more of them than y does.
+template <int R, bool TURNED>
 __global__ void __launch_bounds__(32 * L_WARPS) ns_f32_linear_kernel(const LinearF32Args a)
 {
     extern __shared__ float4 linear_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* rows_smem = reinterpret_cast<float*>(linear_smem);              // [8 R][k]
     float* ring = rows_smem + (size_t)R * L_WARPS * a.k;                  // [L_STAGES][LK][L_LD]
-    const int col0 = (int)(a.turned ? blockIdx.y : blockIdx.x) * LT, row0 = ((int)(a.turned ? blockIdx.x : blockIdx.y) * L_WARPS + warp) * R;
+    const int col0 = (TURNED ? blockIdx.y : blockIdx.x) * LT, row0 = ((TURNED ? blockIdx.x : blockIdx.y) * L_WARPS + warp) * R;
     const int slices = (a.k + LK - 1) / LK;
 
     auto load_w = [&](int slice) {
@@ -297,21 +297,25 @@ __global__ void ns_f32_embed_positions_kernel(const float* __restrict__ ids, con
         if (_rc != NS_OK) return _rc;        \
     }
 
-template <int R>
-static int launch_linear(NsDevice* d, LinearF32Args a)
+template <int R, bool TURNED>
+static int launch_linear_as(NsDevice* d, const LinearF32Args& a, dim3 grid)
 {
     constexpr int ring = L_STAGES * LK * L_LD * (int)sizeof(float);
     static bool configured[64] = {false};
     if (!configured[d->ordinal]) {
-        NS_CUDA(cudaFuncSetAttribute(ns_f32_linear_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, LINEAR_A_BYTES + ring));
+        NS_CUDA(cudaFuncSetAttribute(ns_f32_linear_kernel<R, TURNED>, cudaFuncAttributeMaxDynamicSharedMemorySize, LINEAR_A_BYTES + ring));
         configured[d->ordinal] = true;
     }
-    const unsigned across = (unsigned)(((int64_t)a.n + LT - 1) / LT), down = (unsigned)(((int64_t)a.m + L_WARPS * R - 1) / (L_WARPS * R));
-    a.turned = down > 65535;
-    NS_REQUIRE(!a.turned || across <= 65535, NS_ERR_ARGUMENT, "ns_f32_linear: %d x %d is too large", a.m, a.n);
-    const dim3 grid = a.turned ? dim3(down, across) : dim3(across, down);
-    NS_CUDA(ns_launch_pdl(ns_f32_linear_kernel<R>, grid, dim3(32 * L_WARPS), (size_t)R * L_WARPS * a.k * 4 + ring, d->stream, a));
+    NS_CUDA(ns_launch_pdl(ns_f32_linear_kernel<R, TURNED>, grid, dim3(32 * L_WARPS), (size_t)R * L_WARPS * a.k * 4 + ring, d->stream, a));
     return NS_OK;
+}
+template <int R>
+static int launch_linear(NsDevice* d, const LinearF32Args& a)
+{
+    const unsigned across = (unsigned)(((int64_t)a.n + LT - 1) / LT), down = (unsigned)(((int64_t)a.m + L_WARPS * R - 1) / (L_WARPS * R));
+    if (down <= 65535) return launch_linear_as<R, false>(d, a, dim3(across, down));
+    NS_REQUIRE(across <= 65535, NS_ERR_ARGUMENT, "ns_f32_linear: %d x %d is too large", a.m, a.n);
+    return launch_linear_as<R, true>(d, a, dim3(down, across));
 }
 
 extern "C" int ns_f32_linear(ns_device_t h, uint64_t x, uint64_t gamma, uint64_t beta, float eps, uint64_t w, uint64_t bias, uint64_t residual, int gelu,

@@ -84,7 +84,6 @@ __global__ void __launch_bounds__(256) ns_rms_rows_kernel(const RmsArgs a)
     float* buf = reinterpret_cast<float*>(rms_row4);
     __shared__ float red[8];
     ns_pdl_wait();
-    ns_pdl_trigger();
     // asked for now, read after the reduction (see ns_rms_post_rows_vec_kernel)
     if (VEC && SLABS != NS_ONE_SLAB && a.w != nullptr)
         for (int c = threadIdx.x * 32; c < a.cols; c += blockDim.x * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.w + c));
@@ -111,6 +110,7 @@ __global__ void __launch_bounds__(256) ns_rms_rows_kernel(const RmsArgs a)
             buf[c] = v;
         }
     }
+    ns_pdl_trigger();       // not before the row is here (see ns_rms_post_rows_vec_kernel)
     if (a.w == nullptr) return;
     ss = ns_cta_sum(ss, red);
     const float inv = 1.0f / sqrtf(ss / (float)a.cols + a.eps);
@@ -144,7 +144,6 @@ __global__ void __launch_bounds__(256) ns_rms_post_rows_vec_kernel(const PostRms
     const RmsArgs& a = p.r;
     __shared__ float red[2][8];
     ns_pdl_wait();
-    ns_pdl_trigger();
     const int row = blockIdx.x;
     const int64_t base = (int64_t)row * a.cols;
     float4 s[Q], x[Q], pw[EARLY ? Q : 1], nw[EARLY ? Q : 1];
@@ -175,6 +174,9 @@ __global__ void __launch_bounds__(256) ns_rms_post_rows_vec_kernel(const PostRms
 #pragma unroll
     for (int i = 0; i < Q; i++) { ss = fmaf(s[i].x, s[i].x, ss); ss = fmaf(s[i].y, s[i].y, ss); ss = fmaf(s[i].z, s[i].z, ss); ss = fmaf(s[i].w, s[i].w, ss); }
     const float post = 1.0f / sqrtf(ns_cta_sum(ss, red[0]) / (float)a.cols + a.eps);
+    // The product that follows starts at this signal and asks for its first weights, up to 19 MB.  Given before this row has arrived, the
+    // row's loads (the norms' weights come from HBM) queue behind them: 5.1 us against 3.6 for seven rows of 2048.
+    ns_pdl_trigger();
     ss = 0.0f;
 #pragma unroll
     for (int i = 0; i < Q; i++) {

@@ -60,6 +60,11 @@ int ns_gemv_i8_run(NsDevice* d, const NsGemmParams& p, const void* a, const void
 bool ns_stream_i8_fits(int M, int K);
 int ns_stream_i8_run(NsDevice* d, const NsGemmParams& p, const void* a, const void* w);
 
+// The streaming bf16 kernel (ns_stream_bf16.cu): weights [N, K], one launch, K summed inside the CTA.  `p` must hold M, N, K, the epilogue
+// fields and out (float or bf16).
+bool ns_stream_bf16_fits(const NsDevice* d, int M, int N, int K);
+int ns_stream_bf16_run(NsDevice* d, const NsGemmParams& p, const void* a, const void* w);
+
 #ifdef __CUDACC__
 __device__ __forceinline__ float ns_gemm_residual(const NsGemmParams& p, size_t idx)
 {

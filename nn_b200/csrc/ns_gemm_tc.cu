@@ -1092,6 +1092,21 @@ int ns_gemm_run(NsDevice* d, int kind, const void* a, const void* b, bool b_is_k
     if (stream_env == 1 && kind == NS_KIND_I8 && !deferred && tail == nullptr && d->force_bn == 0 && d->force_splits == 0 && ns_stream_i8_fits(M, K) &&
         ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0)
         return ns_stream_i8_run(d, p, a, b);
+    // Few rows of bf16 against [N, K] weights: the streaming kernel, one slab when the epilogue is deferred.
+    if (kind == NS_KIND_BF16 && !b_is_kn && d->force_bn == 0 && d->force_splits == 0 && ns_stream_bf16_fits(d, M, N, K) &&
+        ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0) {
+        if (deferred) {
+            void* slab = nullptr;
+            int rc = ns_scratch_reserve(d, (size_t)M * N * 4, &slab);
+            if (rc != NS_OK) return rc;
+            p.out = slab;
+            p.out_dtype = NS_F32;
+            p.epilogue = NS_EPI_NONE;
+            *deferred_partial = slab;
+            *deferred_splits = 1;
+        }
+        return ns_stream_bf16_run(d, p, a, b);
+    }
     p.k_blocks = (int)(((int64_t)K * elsize + BKB - 1) / BKB);
     int bn, splits;
     ns_gemm_choose_tiling(d, M, N, p.k_blocks, &bn, &splits, b_is_kn);

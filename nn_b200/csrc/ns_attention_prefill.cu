@@ -1,14 +1,7 @@
-// Causal attention forward for a whole sequence (prefill), head_dim 128, bf16 in / bf16 out, on the
-// sm_100a tensor cores: S = Q.K^T and O += P.V are tcgen05.mma with accumulators in tensor memory,
-// Q/K/V tiles arrive by TMA, the softmax is computed online (running maximum and sum per row) so the
-// [T, T] score tensor never exists.
-//
-// Reference path: MultiHeadAttention.ForwardCore (src/NeuralSharp/Layers/Attention.cs:46-91): three
-// narrow+permute copies, matmul_f32 (Q.K^T) into a [N*H, T, T] tensor, scale_mask_softmax_f32 with an
-// additive -1e9 mask (one thread per row, PtxKernels.Decoding.cs:24-58), matmul_f32 (P.V), permute back.
-// Skipping the key blocks above the diagonal is exact: exp(-1e9 - max) is 0 in float.  The head
-// split/merge copies disappear because the tensor maps take the (batch, head, position) strides of
-// the caller's buffers.
+// Attention of a prompt's portion over the rings of a sliding window (ns_window_prefill; ns_window.cu has the rings and the form for few
+// tokens), bf16 in / bf16 out, on the sm_100a tensor cores: S = Q.K^T and O += P.V are tcgen05.mma with accumulators in tensor
+// memory, Q/K/V tiles arrive by TMA, the softmax is computed online (running maximum and sum per row), so no score tensor exists.
+// Whole sequences without a window: ns_attention_prompt.cu.
 //
 // One persistent CTA per SM draws (batch, head, 128 query rows) tiles from a global counter (tiles of one head adjacent,
 // heavy tiles first); tensor memory and barriers are set up once, and the next tile's Q and first K blocks are loaded
@@ -31,11 +24,9 @@
 // Tensor memory: S_0 at columns [0,128), S_1 at [128,256), O_0 at [256,384), O_1 at [384,512).
 // Every mbarrier wait is bounded; a wait that runs out reports a status code and the CTA leaves.
 //
-// The same kernel serves a portion of a prompt against the rings of a sliding window (ns_window_prefill; ns_window.cu has the rings and
-// the form for few tokens): key blocks are then the 128 positions from a multiple of 128 on, only those that the window of
-// one of the tile's rows reaches are walked, several query heads may share a key/value head, heads have up to 128 columns (the
-// maps fill the rest with zeros; up to 64 use one half), and where the two groups' results are merged a row's sink joins its
-// sum and its gate its result.
+// Key blocks are the 128 positions from a multiple of 128 on; only those that the window of one of the tile's rows reaches are
+// walked.  Several query heads may share a key/value head, heads have up to 128 columns (the maps fill the rest with zeros; up to 64
+// use one half), and where the two groups' results are merged a row's sink joins its sum and its gate its result.
 #include <math.h>
 
 #include "ns_common.cuh"
@@ -50,11 +41,10 @@ constexpr uint32_t FA_SMEM_BYTES = 1024 + 7 * FA_TILE_BYTES + 256;  // Q, 2 x (K
 
 struct FaParams {
     int batch, heads, seq;
-    int causal;
     float scale_log2;  // scale * log2(e)
     int* status;
     int* tile_counter; // zeroed before the launch: CTAs draw their tiles from it in order
-    // windowed form: seq counts the portion's tokens, which follow pos[slots[b]] earlier ones
+    // seq counts the portion's tokens, which follow pos[slots[b]] earlier ones
     int window, ring_len, kv_share;   // kv_share: query heads per key/value head
     const int32_t* slots;
     const int32_t* pos;
@@ -89,9 +79,8 @@ enum { BAR_Q = 0, BAR_Q_FREE = 1, BAR_K0 = 2, BAR_V0 = 4, BAR_K_EMPTY0 = 6, BAR_
 // but the first reader hit in L2, and whichever CTA is free takes the next tile, so the CTAs finish together.
 struct FaTile {
     int b, h, q0, n_blocks;
-    int pos0, j0;      // windowed form: the sequence's earlier tokens, the first key block
+    int pos0, j0;      // the sequence's earlier tokens, the first key block
 };
-template <bool WINDOW>
 __device__ __forceinline__ void fa_tile(const FaParams& p, int n_qt, int idx, FaTile& t)
 {
     const int qt = n_qt - 1 - idx % n_qt;
@@ -99,8 +88,6 @@ __device__ __forceinline__ void fa_tile(const FaParams& p, int n_qt, int idx, Fa
     t.b = bh / p.heads;
     t.h = bh % p.heads;
     t.q0 = qt * FA_BLOCK;
-    t.n_blocks = p.causal ? qt + 1 : n_qt;
-    if (WINDOW) t.j0 = 0;
 }
 // the key blocks that the windows of the tile's rows reach
 __device__ __forceinline__ void fa_window(const FaParams& p, int pos0, FaTile& t)
@@ -111,7 +98,7 @@ __device__ __forceinline__ void fa_window(const FaParams& p, int pos0, FaTile& t
 }
 
 // KH, VH: 64-column halves of a query / key and of a value
-template <int KH, int VH, bool WINDOW>
+template <int KH, int VH>
 __global__ void __launch_bounds__(FA_THREADS, 1) ns_attention_prefill_kernel(const __grid_constant__ FaMaps maps, const FaParams p)
 {
     extern __shared__ uint8_t smem_raw[];
@@ -136,18 +123,11 @@ __global__ void __launch_bounds__(FA_THREADS, 1) ns_attention_prefill_kernel(con
     const uint32_t tile_ring = bar_base + 8u * BAR_COUNT + 16u;
     auto next_tile = [&](int it, FaTile& t) {
         if (!ns_mbar_wait(bar(BAR_TILE0 + (it & 3)), (it >> 2) & 1, abort_flag, p.status, 300 + 11)) return false;
-        int idx;
-        if (WINDOW) {
-            int pos0;
-            asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(idx), "=r"(pos0) : "r"(tile_ring + 8u * (it & 3)) : "memory");
-            if (idx < 0) return false;
-            fa_tile<WINDOW>(p, n_qt, idx, t);
-            fa_window(p, pos0, t);
-            return true;
-        }
-        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(idx) : "r"(tile_ring + 4u * (it & 3)) : "memory");
+        int idx, pos0;
+        asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(idx), "=r"(pos0) : "r"(tile_ring + 8u * (it & 3)) : "memory");
         if (idx < 0) return false;
-        fa_tile<WINDOW>(p, n_qt, idx, t);
+        fa_tile(p, n_qt, idx, t);
+        fa_window(p, pos0, t);
         return true;
     };
 
@@ -196,9 +176,9 @@ __global__ void __launch_bounds__(FA_THREADS, 1) ns_attention_prefill_kernel(con
         if (lane == 0) {
             // where block j's rows, and the head, lie in the maps
             int slot = 0, pos0 = 0, seq_now = -1;
-            auto key_row = [&](const FaTile& t, int j) { return WINDOW ? (t.j0 + j) * FA_BLOCK % p.ring_len : j * FA_BLOCK; };
+            auto key_row = [&](const FaTile& t, int j) { return (t.j0 + j) * FA_BLOCK % p.ring_len; };
             auto load_k = [&](const FaTile& t, int j, int gj) {
-                const int s = gj & 1, y = key_row(t, j), z = WINDOW ? t.h / p.kv_share : t.h, w = WINDOW ? slot : t.b;
+                const int s = gj & 1, y = key_row(t, j), z = t.h / p.kv_share, w = slot;
                 if (gj >= 2 && !ns_mbar_wait(bar(BAR_K_EMPTY0 + s), ((gj >> 1) - 1) & 1, abort_flag, p.status, code + 1)) return false;
                 ns_mbar_expect_tx(bar(BAR_K0 + s), KH * FA_HALF_BYTES);
 #pragma unroll
@@ -206,7 +186,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) ns_attention_prefill_kernel(con
                 return true;
             };
             auto load_v = [&](const FaTile& t, int j, int gj) {
-                const int s = gj & 1, y = key_row(t, j), z = WINDOW ? t.h / p.kv_share : t.h, w = WINDOW ? slot : t.b;
+                const int s = gj & 1, y = key_row(t, j), z = t.h / p.kv_share, w = slot;
                 if (gj >= 2 && !ns_mbar_wait(bar(BAR_V_EMPTY0 + s), ((gj >> 1) - 1) & 1, abort_flag, p.status, code + 1)) return false;
                 ns_mbar_expect_tx(bar(BAR_V0 + s), VH * FA_HALF_BYTES);
 #pragma unroll
@@ -221,23 +201,18 @@ __global__ void __launch_bounds__(FA_THREADS, 1) ns_attention_prefill_kernel(con
                 if (it > 0) ok = ns_mbar_wait(bar(BAR_Q_FREE), (it - 1) & 1, abort_flag, p.status, code + 1);
                 if (!ok) break;
                 const int idx = atomicAdd(p.tile_counter, 1);
-                if (WINDOW) {
-                    if (idx < total) {
-                        fa_tile<WINDOW>(p, n_qt, idx, t);
-                        if (t.b != seq_now) {            // the tiles of a sequence follow one another
-                            seq_now = t.b;
-                            slot = p.slots[t.b];
-                            pos0 = p.pos[slot];
-                        }
-                        fa_window(p, pos0, t);
+                if (idx < total) {
+                    fa_tile(p, n_qt, idx, t);
+                    if (t.b != seq_now) {            // the tiles of a sequence follow one another
+                        seq_now = t.b;
+                        slot = p.slots[t.b];
+                        pos0 = p.pos[slot];
                     }
-                    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(tile_ring + 8u * (it & 3)), "r"(idx < total ? idx : -1), "r"(pos0) : "memory");
-                } else {
-                    asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile_ring + 4u * (it & 3)), "r"(idx < total ? idx : -1) : "memory");
+                    fa_window(p, pos0, t);
                 }
+                asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(tile_ring + 8u * (it & 3)), "r"(idx < total ? idx : -1), "r"(pos0) : "memory");
                 ns_mbar_arrive(bar(BAR_TILE0 + (it & 3)));
                 if (idx >= total) break;
-                if (!WINDOW) fa_tile<WINDOW>(p, n_qt, idx, t);
                 ns_mbar_expect_tx(bar(BAR_Q), KH * FA_HALF_BYTES);
 #pragma unroll
                 for (int i = 0; i < KH; i++) ns_tma_load_4d(q_smem + i * FA_HALF_BYTES, &maps.q, bar(BAR_Q), i * 64, t.q0, t.h, t.b);
@@ -353,7 +328,7 @@ __global__ void __launch_bounds__(FA_THREADS, 1) ns_attention_prefill_kernel(con
         int kg = 0;                               // blocks this group has handled so far, over all tiles
         FaTile t;
         for (int it = 0; ok && next_tile(it, t); it++) {
-            const int qi = WINDOW ? t.pos0 + t.q0 + r : t.q0 + r;   // absolute query position
+            const int qi = t.pos0 + t.q0 + r;   // absolute query position
             float m_ref = -INFINITY;             // reference maximum of this group's blocks of the tile (raw score units)
             float l_run = 0.0f;                  // sum of this group's exponentials relative to m_ref
             int n_mine = 0;
@@ -375,18 +350,16 @@ __global__ void __launch_bounds__(FA_THREADS, 1) ns_attention_prefill_kernel(con
                 }
                 ns_tc_fence_before();
                 ns_mbar_arrive(bar(BAR_S_FREE0 + g));
-                // mask: keys after the query (causal) or past the end of the sequence
-                // windowed form: or more than the window before it (what a ring holds past a row's own position is later than it)
-                const int kv0 = (WINDOW ? t.j0 + j : j) * FA_BLOCK;
-                const bool need_mask = WINDOW ? kv0 + 127 > t.pos0 + t.q0 || kv0 <= t.pos0 + t.q0 + 127 - p.window
-                                              : (p.causal && kv0 + 127 > t.q0) || kv0 + 128 > p.seq;
+                // mask: keys after the query or more than the window before it (what a ring holds past a row's own position is later than it)
+                const int kv0 = (t.j0 + j) * FA_BLOCK;
+                const bool need_mask = kv0 + 127 > t.pos0 + t.q0 || kv0 <= t.pos0 + t.q0 + 127 - p.window;
                 float mx;
                 if (need_mask) {
                     mx = -INFINITY;
 #pragma unroll
                     for (int c = 0; c < 128; c++) {
                         const int kj = kv0 + c;
-                        const bool dead = WINDOW ? kj > qi || kj <= qi - p.window : (p.causal && kj > qi) || kj >= p.seq;
+                        const bool dead = kj > qi || kj <= qi - p.window;
                         if (dead) sb[c] = 0xFF800000u;  // -inf
                         mx = fmaxf(mx, __uint_as_float(sb[c]));
                     }
@@ -481,15 +454,13 @@ __global__ void __launch_bounds__(FA_THREADS, 1) ns_attention_prefill_kernel(con
                 float a_mine = m_ref == -INFINITY ? 0.0f : fa_exp2((m_ref - m_all) * p.scale_log2);
                 float a_other = m_o == -INFINITY ? 0.0f : fa_exp2((m_o - m_all) * p.scale_log2);
                 float l_sink = 0.0f, row_gate = 1.0f;
-                if (WINDOW) {
-                    if (p.sink != nullptr) {
-                        const float s = p.sink[t.h] * 1.4426950408889634f, m2 = m_all * p.scale_log2, top = fmaxf(m2, s), f = fa_exp2(m2 - top);
-                        l_sink = fa_exp2(s - top);
-                        a_mine *= f;
-                        a_other *= f;
-                    }
-                    if (p.gate != nullptr) row_gate = t.q0 + r < p.seq ? p.gate[((int64_t)t.b * p.seq + t.q0 + r) * p.heads + t.h] : 0.0f;
+                if (p.sink != nullptr) {
+                    const float s = p.sink[t.h] * 1.4426950408889634f, m2 = m_all * p.scale_log2, top = fmaxf(m2, s), f = fa_exp2(m2 - top);
+                    l_sink = fa_exp2(s - top);
+                    a_mine *= f;
+                    a_other *= f;
                 }
+                if (p.gate != nullptr) row_gate = t.q0 + r < p.seq ? p.gate[((int64_t)t.b * p.seq + t.q0 + r) * p.heads + t.h] : 0.0f;
                 // Which group got the tile's even-numbered key blocks depends on how many blocks this CTA has walked before
                 // (tiles are drawn from a counter at run time).  The result must not: the two partial results are combined
                 // in the order (even blocks, odd blocks) of the TILE, whichever group holds which, with every rounding spelt out.
@@ -497,9 +468,9 @@ __global__ void __launch_bounds__(FA_THREADS, 1) ns_attention_prefill_kernel(con
                 const float l_even = mine_even ? l_run : l_o, a_even = mine_even ? a_mine : a_other;
                 const float l_odd = mine_even ? l_o : l_run, a_odd = mine_even ? a_other : a_mine;
                 float l_tot = __fadd_rn(__fmul_rn(l_even, a_even), __fmul_rn(l_odd, a_odd));
-                if (WINDOW) l_tot = __fadd_rn(l_tot, l_sink);
+                l_tot = __fadd_rn(l_tot, l_sink);
                 float inv = l_tot > 0.0f ? 1.0f / l_tot : 0.0f;
-                if (WINDOW) inv *= row_gate;
+                inv *= row_gate;
                 const float w_even = __fmul_rn(a_even, inv), w_odd = __fmul_rn(a_odd, inv);
                 const uint32_t o_mine = lane_addr + 256 + g * 128, o_other = lane_addr + 256 + (g ^ 1) * 128;
                 // group g finishes output dims [64 g, 64 g + 64): (O_mine w_mine + O_other w_other) -> bf16 -> the upper half of
@@ -574,53 +545,10 @@ int make_map(CUtensorMap* m, uint64_t base, int batch, int heads, int seq, int64
 
 }  // namespace
 
-extern "C" int ns_attention_prefill(ns_device_t h, uint64_t q, uint64_t k, uint64_t v, uint64_t o, int batch, int heads, int seq, int head_dim,
-                                    const int64_t* q_strides, const int64_t* k_strides, const int64_t* v_strides, const int64_t* o_strides,
-                                    float scale, int causal)
-{
-    NsDevice* d = ns_dev(h);
-    int rc = ns_device_make_current(d);
-    if (rc != NS_OK) return rc;
-    NS_REQUIRE(q && k && v && o && q_strides && k_strides && v_strides && o_strides, NS_ERR_ARGUMENT, "ns_attention_prefill: null argument");
-    NS_REQUIRE(head_dim == 128, NS_ERR_ARGUMENT, "ns_attention_prefill: head_dim must be 128 (got %d)", head_dim);
-    NS_REQUIRE(batch > 0 && heads > 0 && seq > 0, NS_ERR_ARGUMENT, "ns_attention_prefill: bad shape");
-    const int n_qt = (seq + FA_BLOCK - 1) / FA_BLOCK;
-    NS_REQUIRE((int64_t)batch * heads * n_qt < (1LL << 31), NS_ERR_ARGUMENT, "ns_attention_prefill: too many tiles");
-    FaMaps maps;
-    rc = make_map(&maps.q, q, batch, heads, seq, q_strides[0], q_strides[1], q_strides[2], 128);
-    if (rc == NS_OK) rc = make_map(&maps.k, k, batch, heads, seq, k_strides[0], k_strides[1], k_strides[2], 128);
-    if (rc == NS_OK) rc = make_map(&maps.v, v, batch, heads, seq, v_strides[0], v_strides[1], v_strides[2], 128);
-    if (rc == NS_OK) rc = make_map(&maps.o, o, batch, heads, seq, o_strides[0], o_strides[1], o_strides[2], 32);
-    if (rc != NS_OK) return rc;
-    // the tile counter: one word at the start of the device object's scratch block, zeroed in stream order
-    void* counter = nullptr;
-    rc = ns_scratch_reserve(d, 256, &counter);
-    if (rc != NS_OK) return rc;
-    NS_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), d->stream));
-    FaParams p;
-    p.tile_counter = reinterpret_cast<int*>(counter);
-    p.batch = batch; p.heads = heads; p.seq = seq; p.causal = causal ? 1 : 0;
-    p.scale_log2 = scale * 1.4426950408889634f;
-    p.status = d->status_dev;
-    p.window = p.ring_len = p.kv_share = 0;
-    p.slots = p.pos = nullptr;
-    p.sink = p.gate = nullptr;
-    static bool configured[64] = {false};
-    if (!configured[d->ordinal]) {
-        NS_CUDA(cudaFuncSetAttribute(ns_attention_prefill_kernel<2, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FA_SMEM_BYTES));
-        configured[d->ordinal] = true;
-    }
-    // persistent: one CTA per SM walks its share of the (batch, head, query tile) list
-    const int total = batch * heads * n_qt;
-    ns_attention_prefill_kernel<2, 2, false><<<total < d->sm_count ? total : d->sm_count, FA_THREADS, FA_SMEM_BYTES, d->stream>>>(maps, p);
-    NS_CUDA(cudaGetLastError());
-    return NS_OK;
-}
-
 template <int KH, int VH>
 static int launch_window(NsDevice* d, const FaMaps& maps, const FaParams& p, int total)
 {
-    auto k = ns_attention_prefill_kernel<KH, VH, true>;
+    auto k = ns_attention_prefill_kernel<KH, VH>;
     NS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FA_SMEM_BYTES));
     k<<<total < d->sm_count ? total : d->sm_count, FA_THREADS, FA_SMEM_BYTES, d->stream>>>(maps, p);
     NS_CUDA(cudaGetLastError());
@@ -656,7 +584,7 @@ extern "C" int ns_window_prefill(ns_device_t h, uint64_t q, uint64_t k_ring, uin
     NS_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), d->stream));
     FaParams p;
     p.tile_counter = reinterpret_cast<int*>(counter);
-    p.batch = batch; p.heads = heads; p.seq = steps; p.causal = 1;
+    p.batch = batch; p.heads = heads; p.seq = steps;
     p.scale_log2 = scale * 1.4426950408889634f;
     p.status = d->status_dev;
     p.window = window; p.ring_len = ring_len; p.kv_share = heads / kv_heads;

@@ -125,3 +125,21 @@ def test_results_do_not_depend_on_the_tile_schedule(dev, orc):
         outs.append(o.download())
         o.release()
     assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[0], outs[2])
+
+
+@pytest.mark.parametrize("S", [1, 127, 128, 129, 255, 256, 257, 384, 511, 513, 1000])
+@pytest.mark.parametrize("causal", [True, False])
+def test_tiles_of_one_group_and_of_two(dev, orc, S, causal):
+    """Where every 128 query rows get an SM of their own a tile is one group's, else two groups' (one without rows where S leaves fewer than 129):
+    a row's result is the same to the bit, and within bf16 of the oracle.  Scores grow along the sequence, so the reference maximum moves."""
+    heads, scale = 2, 0.2
+    many = 200 // heads                                              # 200 tiles of 128 rows are more than a B200 has SMs
+    grow = np.linspace(0.3, 2.0, S, dtype=np.float32)[:, None]
+    q, k, v = (orc.round_bf16(orc.normal((1, heads, S, DH), 20 + i) * (grow if i == 1 else 1)) for i in range(3))
+    one = _run_bhsd(dev, q, k, v, 1, heads, S, scale, causal)
+    all_ = _run_bhsd(dev, *(np.repeat(x, many, 0) for x in (q, k, v)), many, heads, S, scale, causal)
+    assert np.array_equal(all_, np.repeat(one, many, 0))
+    for h in range(heads):
+        exp = orc.attention_slice(*(orc.widen_bf16(x[0, h]) for x in (q, k, v)), 0, scale, causal)
+        got = orc.widen_bf16(one[0, h])
+        assert orc.close(orc.bf16_round_trip(exp), got, TOL), (h, orc.max_err(exp, got))

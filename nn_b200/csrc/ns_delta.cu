@@ -69,7 +69,29 @@ NS_DEVINL void conv_load(const NsSource& s, int64_t idx, float (&x)[V])
     }
 }
 
-template <typename T, int V, int TAPS, int SRC>
+// The sums of v[0..8) over the warp, in the order ns_warp_sum takes: lane l has that of v[l / 4].
+NS_DEVINL float conv_sum8(float (&v)[8], int lane)
+{
+#pragma unroll
+    for (int o = 16, half = 4; half > 0; o >>= 1, half >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < half; i++) {
+            const float send = up ? v[i] : v[i + half], keep = up ? v[i + half] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    float r = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 2);
+    return r + __shfl_xor_sync(0xffffffffu, r, 1);
+}
+
+// PIECE: tokens whose inputs are in registers together (8; 1 for a step of one token, whose loads are then all there is).  What bounds a prompt is
+// the arithmetic of a warp, not HBM: the tokens of a piece are computed side by side in place of their inputs, last one first, and the heads' lengths
+// of all eight are summed in one butterfly, so that a lane takes one root and one division where it took eight.
+// Weights of four taps come as one load a channel, and a bf16 matrix a piece ahead.  Against one token after the other (us): 16 x 512 tokens of 4096
+// channels, bf16 in, float out 112 -> 67 (floor 31), of 6144 157 -> 99; one token of 64 sequences, 6144 channels of 3 slabs 10.5 -> 5.2, of 250
+// sequences, 4096 channels of 4 slabs 19.8 -> 10.3; 4 x 100 of 2 slabs 13.4 -> 10.8.  Eight pieces a warp instead of four: 66, 96, but 3 x 300 tokens 28 for 16.
+template <typename T, int V, int TAPS, int PIECE, int SRC>
 __global__ void __launch_bounds__(128) ns_short_conv_slide_kernel(const ConvArgs a, int span, int units, int pieces)
 {
     ns_pdl_wait();
@@ -87,64 +109,93 @@ __global__ void __launch_bounds__(128) ns_short_conv_slide_kernel(const ConvArgs
     const int64_t src0 = (int64_t)b * a.steps * a.src.ld + g.col + ch;
     const int per = CONV_WARP * pieces;
     const int t0 = (span == 4 ? (int)blockIdx.x * 4 + warp : (int)blockIdx.x) * per, t1 = min(t0 + per, a.steps);
-    float w[TAPS][V], x[TAPS][V];      // w[n]: weight of the input n tokens back; x[n]: that input
+    float w[TAPS][V], back[TAPS][V];   // w[n]: weight of the input n tokens back; back[n]: the input n tokens before the piece
+    const bool vec_w = TAPS == 4 && taps == 4 && (reinterpret_cast<uintptr_t>(g.w) & 15) == 0;
 #pragma unroll
-    for (int n = 0; n < TAPS; n++)
+    for (int i = 0; i < V; i++) {
+        float4 wi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (vec_w && mine) wi = __ldg(reinterpret_cast<const float4*>(g.w) + ch + i);
 #pragma unroll
-        for (int i = 0; i < V; i++) {
-            w[n][i] = mine && n < taps ? __ldg(g.w + (int64_t)(ch + i) * taps + taps - 1 - n) : 0.0f;
-            x[n][i] = 0.0f;
+        for (int n = 0; n < TAPS; n++) {
+            back[n][i] = 0.0f;
+            if (vec_w) w[n][i] = n == 0 ? wi.w : (n == 1 ? wi.z : (n == 2 ? wi.y : wi.x));
+            else w[n][i] = mine && n < taps ? __ldg(g.w + (int64_t)(ch + i) * taps + taps - 1 - n) : 0.0f;
         }
+    }
+    // the inputs of a piece: for one bf16 matrix they are asked for a piece ahead, as they lie in memory
+    constexpr bool AHEAD = SRC == CONV_BF16 && V == 4;
+    uint2 next[AHEAD ? PIECE : 1];
+    auto ask = [&](int tp) {
+        if constexpr (AHEAD) {
+#pragma unroll
+            for (int j = 0; j < PIECE; j++)
+                next[j] = mine && tp + j < t1 ? *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(a.src.ptr) + src0 + (int64_t)(tp + j) * a.src.ld) : make_uint2(0, 0);
+        }
+    };
+    ask(t0);
     if (mine && t0 < t1) {
-        // x[n - 1] becomes x[n] before the first token is loaded
 #pragma unroll
         for (int n = 1; n < TAPS; n++) {
             const int tt = t0 - n;
-            if (n >= taps || pos0 + tt < 0) continue;
+            if (n >= taps) continue;
             if (tt >= 0) {
-                conv_load<V, SRC>(a.src, src0 + (int64_t)tt * a.src.ld, x[n - 1]);
-            } else {
+                conv_load<V, SRC>(a.src, src0 + (int64_t)tt * a.src.ld, back[n]);
+            } else if (pos0 + tt >= 0) {
                 const float* p = hist + (int64_t)((pos0 + tt) % taps) * channels;
 #pragma unroll
-                for (int i = 0; i < V; i++) x[n - 1][i] = p[i];
+                for (int i = 0; i < V; i++) back[n][i] = p[i];
             }
         }
     }
-    for (int tp = t0; tp < t1; tp += CONV_WARP) {
+    for (int tp = t0; tp < t1; tp += PIECE) {
         // all inputs of a piece are on their way before the first is used
-        float in[CONV_WARP][V];
+        float in[PIECE][V], ss[PIECE], last[TAPS][V];
 #pragma unroll
-        for (int j = 0; j < CONV_WARP; j++)
-            if (mine && tp + j < t1) conv_load<V, SRC>(a.src, src0 + (int64_t)(tp + j) * a.src.ld, in[j]);
+        for (int j = 0; j < PIECE; j++) {
 #pragma unroll
-        for (int j = 0; j < CONV_WARP; j++) {
-            const int t = tp + j;
-            if (t >= t1) break;
+            for (int i = 0; i < V; i++) in[j][i] = 0.0f;
+            if constexpr (AHEAD) {
+                in[j][0] = __uint_as_float(next[j].x << 16); in[j][1] = __uint_as_float(next[j].x & 0xFFFF0000u);
+                in[j][2] = __uint_as_float(next[j].y << 16); in[j][3] = __uint_as_float(next[j].y & 0xFFFF0000u);
+            } else if (mine && tp + j < t1) conv_load<V, SRC>(a.src, src0 + (int64_t)(tp + j) * a.src.ld, in[j]);
+        }
+        if (tp + PIECE < t1) ask(tp + PIECE);
+        auto input = [&](int j, int i) { return j >= 0 ? in[j < 0 ? 0 : j][i] : back[j < 0 ? -j : 0][i]; };
 #pragma unroll
-            for (int n = TAPS - 1; n > 0; n--)
+        for (int n = 1; n < TAPS; n++)
 #pragma unroll
-                for (int i = 0; i < V; i++) x[n][i] = x[n - 1][i];
+            for (int i = 0; i < V; i++) last[n][i] = input(PIECE - n, i);
 #pragma unroll
-            for (int i = 0; i < V; i++) x[0][i] = mine ? in[j][i] : 0.0f;
-            float y[V], ss = 0.0f;
+        for (int j = PIECE - 1; j >= 0; j--) {
+            ss[j] = 0.0f;
 #pragma unroll
             for (int i = 0; i < V; i++) {
                 float acc = 0.0f;
 #pragma unroll
-                for (int n = TAPS - 1; n >= 0; n--) acc = fmaf(x[n][i], w[n][i], acc);
-                y[i] = mine ? __fdividef(acc, 1.0f + expf(-acc)) : 0.0f;
-                ss = fmaf(y[i], y[i], ss);
+                for (int n = TAPS - 1; n >= 0; n--) acc = fmaf(input(j - n, i), w[n][i], acc);
+                in[j][i] = mine ? __fdividef(acc, 1.0f + expf(-acc)) : 0.0f;
+                ss[j] = fmaf(in[j][i], in[j][i], ss[j]);
             }
-            float f = 1.0f;
-            if (g.unit) f = g.scale / sqrtf(ns_warp_sum(ss) + 1e-6f);
-            if (mine) {
-                T* out = reinterpret_cast<T*>(g.out) + ((int64_t)b * a.steps + t) * g.out_ld + ch;
-                if constexpr (V == 4) {
-                    ns_store4(out, make_float4(y[0] * f, y[1] * f, y[2] * f, y[3] * f));
-                } else {
+        }
 #pragma unroll
-                    for (int i = 0; i < V; i++) ns_store(out + i, y[i] * f);
-                }
+        for (int n = 1; n < TAPS; n++)
+#pragma unroll
+            for (int i = 0; i < V; i++) back[n][i] = last[n][i];
+        float f = 1.0f;
+        if (g.unit) {
+            if constexpr (PIECE == 8) f = g.scale / sqrtf(conv_sum8(ss, lane) + 1e-6f);
+            else f = g.scale / sqrtf(ns_warp_sum(ss[0]) + 1e-6f);
+        }
+#pragma unroll
+        for (int j = 0; j < PIECE; j++) {
+            const float fj = PIECE == 8 ? __shfl_sync(0xffffffffu, f, j * 4) : f;
+            if (!mine || tp + j >= t1) continue;
+            T* out = reinterpret_cast<T*>(g.out) + ((int64_t)b * a.steps + tp + j) * g.out_ld + ch;
+            if constexpr (V == 4) {
+                ns_store4(out, make_float4(in[j][0] * fj, in[j][1] * fj, in[j][2] * fj, in[j][3] * fj));
+            } else {
+#pragma unroll
+                for (int i = 0; i < V; i++) ns_store(out + i, in[j][i] * fj);
             }
         }
     }
@@ -565,20 +616,23 @@ extern "C" int ns_short_conv(ns_device_t h, uint64_t src, int splits, int src_dt
             NS_CUDA(ns_launch_plain(k, sgrid, dim3(128), 0, d->stream, a, span, units, pieces));
             return NS_OK;
         };
-        // Slabs together, except where four channels a lane of four taps (146 registers against 128: three CTAs a SM, not four) need a second wave.
-        // Together against in turn (us): 32 heads of 128, 4 taps, 7 tokens of 8 slabs 3.9, 4.2; 64 of 4 slabs 9.0, 6.2; 250 of 4 slabs
-        // 12.4, 14.1; 6 taps, 64 tokens of 4 slabs 9.6, 10.1, 4 x 1000 tokens of one 106, 83; heads of 64, 4 taps, 64 of 4 slabs
-        // 4.6, 4.8, 4 x 1000 of one 36, 25.
+        // Slabs together, except where four channels a lane of four taps (more registers, fewer CTAs a SM) need a second wave.  Measured with eight
+        // tokens a piece, together against in turn (us): 32 heads of 128, 4 taps, 7 tokens of 8 slabs 3.9, 4.2; 6 taps, 64 tokens of 4 slabs
+        // 9.6, 10.1, 4 x 1000 tokens of one 106, 83; heads of 64, 4 taps, 64 of 4 slabs 4.6, 4.8, 4 x 1000 of one 36, 25.
         const bool together = splits > 2 && (v < 4 || most_taps > 4 || (int64_t)sgrid.x * sgrid.y * sgrid.z <= 2 * d->sm_count);
         auto pick = [&](auto zero) -> int {
             using T = decltype(zero);
             if (v == 4 && most_taps <= 4 && splits == 1 && steps > CONV_WARP)
-                return src_dtype == NS_F32 ? slide(ns_short_conv_slide_kernel<T, 4, 4, CONV_F32>) : slide(ns_short_conv_slide_kernel<T, 4, 4, CONV_BF16>);
+                return src_dtype == NS_F32 ? slide(ns_short_conv_slide_kernel<T, 4, 4, 8, CONV_F32>) : slide(ns_short_conv_slide_kernel<T, 4, 4, 8, CONV_BF16>);
             auto any = [&](auto source) -> int {
                 constexpr int S = decltype(source)::value;
-                if (most_taps <= 4)
-                    return v == 1 ? slide(ns_short_conv_slide_kernel<T, 1, 4, S>) : (v == 2 ? slide(ns_short_conv_slide_kernel<T, 2, 4, S>) : slide(ns_short_conv_slide_kernel<T, 4, 4, S>));
-                return v == 1 ? slide(ns_short_conv_slide_kernel<T, 1, 8, S>) : (v == 2 ? slide(ns_short_conv_slide_kernel<T, 2, 8, S>) : slide(ns_short_conv_slide_kernel<T, 4, 8, S>));
+                auto of = [&](auto piece) {
+                    constexpr int P = decltype(piece)::value;
+                    if (most_taps <= 4)
+                        return v == 1 ? slide(ns_short_conv_slide_kernel<T, 1, 4, P, S>) : (v == 2 ? slide(ns_short_conv_slide_kernel<T, 2, 4, P, S>) : slide(ns_short_conv_slide_kernel<T, 4, 4, P, S>));
+                    return v == 1 ? slide(ns_short_conv_slide_kernel<T, 1, 8, P, S>) : (v == 2 ? slide(ns_short_conv_slide_kernel<T, 2, 8, P, S>) : slide(ns_short_conv_slide_kernel<T, 4, 8, P, S>));
+                };
+                return steps == 1 ? of(std::integral_constant<int, 1>()) : of(std::integral_constant<int, CONV_WARP>());
             };
             return together ? any(std::integral_constant<int, CONV_SLABS>()) : any(std::integral_constant<int, CONV_ANY>());
         };

@@ -157,6 +157,32 @@ def test_short_convolution_over_cuts(dev, taps, cuts):
         close(g, e, 1e-5)
 
 
+@pytest.mark.parametrize("steps", [1, 8, 9, 31, 32, 33, 257, 300])
+@pytest.mark.parametrize("taps,hd,ragged", [(4, 128, 0), (3, 128, 0), (4, 120, 0), (4, 128, 1)])
+def test_short_convolution_of_one_bf16_matrix(dev, steps, taps, hd, ragged):
+    """A prompt's product as it is: pieces of eight tokens, the next one on its way; a portion's seams and its carried inputs; weights off 16 bytes."""
+    B, heads, before = 3, 2, 5
+    c = heads * hd
+    x = f32(bf16_bits(rng_for(6, steps, taps, hd).standard_normal((B, before + steps, c))))
+    w = rng_for(7, taps, hd).standard_normal((c, taps)).astype(np.float32)
+    src = dev.from_numpy(bf16_bits(x[:, before:].reshape(B * steps, c)))
+    hist = np.zeros((B, taps, c), np.float32)
+    for t in range(before):
+        hist[:, t % taps] = x[:, t]
+    dh, out = dev.from_numpy(hist), dev.empty(B * steps * c)
+    dw = dev.from_numpy(np.concatenate([np.zeros(ragged, np.float32), w.ravel()]))
+    slots, pos = dev.from_numpy(np.arange(B, dtype=np.int32)), dev.from_numpy(np.full(B, before, np.int32))
+    fields = (C.c_int64 * 9)(0, heads, hd, taps, 1, dw.ptr + 4 * ragged, dh.ptr, out.ptr, c)
+    N.call("ns_short_conv", dev.handle, u(src.ptr), 1, N.NS_BF16, c, 1, fields, (C.c_float * 1)(0.25), i64(taps * c), u(slots.ptr), u(pos.ptr), B, steps, N.NS_F32)
+    dev.synchronize()
+    got, after = out.download((B, steps, c)), dh.download((B, taps, c))
+    for i in range(B):
+        want = F.unit(F.short_conv(x[i].astype(np.float64), w.astype(np.float64)).reshape(-1, heads, hd)).reshape(-1, c)[before:] * 0.25
+        close(got[i], want, 1e-5)
+        for t in range(max(0, before + steps - taps + 1), before + steps):
+            assert np.array_equal(after[i, t % taps], x[i, t])
+
+
 # ------------------------------------------------------------------------------------------------ delta rule
 def run_delta(dev, data, cuts, H, kv, dim, vdim, channelwise, slots=(0,), chunk_from=1 << 30):
     """o [B, T, H, vdim] and final states, the sequences fed in `cuts`."""

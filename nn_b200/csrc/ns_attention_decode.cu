@@ -151,14 +151,13 @@ __device__ __forceinline__ void quantize_row_if_last(const DecodeParams& p, int 
 // One CTA per (batch, head, new position, split).  DH = head_dim.  LPR = DH / 32 lanes share one cached row, each
 // lane owning four 16-byte pieces of it (piece i of lane `sub` is piece sub + LPR * i of the row, so the lanes of a
 // row read contiguous 16 * LPR bytes per load).
-template <int DH, int U>
-__global__ void __launch_bounds__(DEC_THREADS) ns_attention_decode_kernel(const DecodeParams p)
+template <int DH, int U, int CTAS>
+__global__ void __launch_bounds__(DEC_THREADS, CTAS) ns_attention_decode_kernel(const DecodeParams p)
 {
     constexpr int LPR = DH / 32;               // lanes per cached row
     constexpr int RPW = 32 / LPR;              // rows per warp per load round
     constexpr int GROUPS = DEC_THREADS / LPR;  // rows in flight per CTA
-    // U = load rounds in flight per lane (a round = one cached row per lane group): two when thousands of CTAs share the
-    // SMs, four when the grid is small and a CTA's own chain of loads is what its time consists of
+    // U = load rounds in flight per lane (a round = one cached row per lane group), CTAS = CTAs an SM the build is held to: see launch_decode
     __shared__ float s_scores[DEC_MAX_CHUNK];
     __shared__ float s_red[DEC_THREADS / 32], s_red2[DEC_THREADS / 32];
     __shared__ float s_acc[GROUPS][DH];
@@ -183,12 +182,15 @@ __global__ void __launch_bounds__(DEC_THREADS) ns_attention_decode_kernel(const 
     // running fold of this CTA's chunks (one CTA per row): thread d < DH holds column d of the weighted values
     float M_run = 0.0f, L_run = 0.0f, O_run = 0.0f;
 
+    // (held to more CTAs an SM, the query is loaded for each chunk and not kept through the values)
+    constexpr bool RELOAD = CTAS > 4;
     float qf[4][8];
-    {
+    auto load_q = [&]() {
         const uint16_t* qrow = p.q + (size_t)(b * p.steps + i) * p.q_stride + h * DH;
 #pragma unroll
         for (int c = 0; c < 4; c++) unpack8(*reinterpret_cast<const uint4*>(qrow + (sub + LPR * c) * 8), qf[c]);
-    }
+    };
+    if (!RELOAD) load_q();
     const int32_t* pt = p.page_table + (size_t)b * p.max_pages;
     const size_t slab = (size_t)p.page_size * DH;
     const size_t head_off = (size_t)h * slab + sub * 8;
@@ -200,11 +202,7 @@ __global__ void __launch_bounds__(DEC_THREADS) ns_attention_decode_kernel(const 
     for (int k = k0; k < k1; k++) {
         const int c0 = k * p.chunk;
         const int c1 = min(kv_len, c0 + p.chunk);
-        float acc[4][8];
-#pragma unroll
-        for (int c = 0; c < 4; c++)
-#pragma unroll
-            for (int d = 0; d < 8; d++) acc[c][d] = 0.0f;
+        if (RELOAD) load_q();
         // ---- scores: s_j = (q . k_j) * scale; U rounds of four loads per lane are in flight before any is used.
         // Loop bounds are uniform per warp because the reduction shuffles need every lane.
         for (int jb = c0 + warp * RPW; jb < c1; jb += (DEC_THREADS / 32) * RPW * U) {
@@ -237,6 +235,24 @@ __global__ void __launch_bounds__(DEC_THREADS) ns_attention_decode_kernel(const 
                 if (sub == 0 && j < c1) s_scores[j - c0] = dot * p.scale;
             }
         }
+        // The first values are asked for before the barriers of the softmax (with that, us: 1024 rows x 576 positions 54.6 -> 53.0, x 100 19.1 -> 18.0,
+        // 1536 x 700 94.5 -> 92.3).
+        uint4 vv[U][4];
+        auto load_values = [&](int jb) {
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int j = jb + u * GROUPS;
+                if (j < c1) {
+                    const uint16_t* vr = row_ptr(p.v_pool, j);
+#pragma unroll
+                    for (int c = 0; c < 4; c++) vv[u][c] = __ldg(reinterpret_cast<const uint4*>(vr + LPR * c * 8));
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 4; c++) vv[u][c] = make_uint4(0, 0, 0, 0);
+                }
+            }
+        };
+        load_values(c0 + grp);
         __syncthreads();
         // ---- the chunk's own maximum and exponentials
         float mx = -INFINITY;
@@ -256,32 +272,25 @@ __global__ void __launch_bounds__(DEC_THREADS) ns_attention_decode_kernel(const 
         __syncthreads();
         sum = s_red2[0] + s_red2[1] + s_red2[2] + s_red2[3];
         // ---- o_g = sum of p_j * v_j over the rows of slot `grp`: rows grp, grp + GROUPS, ... of the chunk
+        float acc[4][8];
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+#pragma unroll
+            for (int d = 0; d < 8; d++) acc[c][d] = 0.0f;
         for (int jb = c0 + grp; jb < c1; jb += GROUPS * U) {
-            uint4 vv[U][4];
-            float pj[U];
 #pragma unroll
             for (int u = 0; u < U; u++) {
                 const int j = jb + u * GROUPS;
-                pj[u] = 0.0f;
-                if (j < c1) {
-                    const uint16_t* vr = row_ptr(p.v_pool, j);
-#pragma unroll
-                    for (int c = 0; c < 4; c++) vv[u][c] = __ldg(reinterpret_cast<const uint4*>(vr + LPR * c * 8));
-                    pj[u] = s_scores[j - c0];
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 4; c++) vv[u][c] = make_uint4(0, 0, 0, 0);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U; u++)
+                const float pj = j < c1 ? s_scores[j - c0] : 0.0f;
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                     float vf[8];
                     unpack8(vv[u][c], vf);
 #pragma unroll
-                    for (int d = 0; d < 8; d++) acc[c][d] = fmaf(pj[u], vf[d], acc[c][d]);
+                    for (int d = 0; d < 8; d++) acc[c][d] = fmaf(pj, vf[d], acc[c][d]);
                 }
+            }
+            load_values(jb + GROUPS * U);
         }
         // ---- the chunk's weighted values: the GROUPS slots summed in slot order
 #pragma unroll
@@ -375,10 +384,20 @@ template <int DH>
 int launch_decode(NsDevice* d, const DecodeParams& p)
 {
     const int rows = p.batch * p.heads * p.steps;
-    if ((int64_t)rows * p.splits < 3 * (int64_t)d->sm_count)   // measured: 384 CTAs gain 9 %, 512 CTAs lose 30 % with four rounds
-        NS_CUDA(ns_launch_plain(ns_attention_decode_kernel<DH, 4>, dim3(rows * p.splits), dim3(DEC_THREADS), 0, d->stream, p));
-    else
-        NS_CUDA(ns_launch_plain(ns_attention_decode_kernel<DH, 2>, dim3(rows * p.splits), dim3(DEC_THREADS), 0, d->stream, p));
+    const int64_t ctas = (int64_t)rows * p.splits;
+    auto cost = [&](int per_sm) { return (ctas + (int64_t)per_sm * d->sm_count - 1) / ((int64_t)per_sm * d->sm_count) * per_sm; };
+    auto launch = [&](auto kernel) -> int {
+        NS_CUDA(ns_launch_plain(kernel, dim3((unsigned)ctas), dim3(DEC_THREADS), 0, d->stream, p));
+        return NS_OK;
+    };
+    // Builds: four CTAs an SM, or five (the query reloaded for each chunk, 96 registers) where that leaves fewer or smaller last waves; four rounds of loads in flight
+    // where a CTA's own chain of loads is what its time consists of (measured: 384 CTAs gain 9 %, 512 lose 30 % with four rounds).  Five against
+    // four an SM, us: 2048 CTAs x 4096 positions 603, 655; 640 x 300 20.6, 28; 1024 x 576 58, 53; 1536 x 700 99, 92.
+    int rc;
+    if (ctas < 3 * (int64_t)d->sm_count) rc = launch(ns_attention_decode_kernel<DH, 4, 3>);
+    else if (cost(5) < cost(4)) rc = launch(ns_attention_decode_kernel<DH, 2, 5>);
+    else rc = launch(ns_attention_decode_kernel<DH, 2, 4>);
+    if (rc != NS_OK) return rc;
     if (p.splits > 1) {
         NS_CUDA(ns_launch_plain(ns_attention_combine_kernel<DH>, dim3(rows), dim3(DH < 64 ? 32 : 64), 0, d->stream, p));
     }

@@ -197,3 +197,28 @@ def test_a_sequence_in_a_batch_equals_the_sequence_in_a_small_batch(dev, orc, ca
         assert np.array_equal(small, big[rows]), f"sequences {rows} differ between a batch of {len(rows)} and a batch of {B}"
     exp = orc.attention_slice(orc.widen_bf16(q[5, :, 3]), orc.widen_bf16(k[5, :, 3]), orc.widen_bf16(v[5, :, 3]), length - 1, scale)
     assert orc.close(orc.bf16_round_trip(exp), orc.widen_bf16(big[5, :, 3]), TOL)
+
+
+@pytest.mark.parametrize("dh", [32, 64, 128])
+@pytest.mark.parametrize("B", [28, 40, 64])      # 448, 640 and 1024 rows of 16 heads: four CTAs an SM, five, four
+@pytest.mark.parametrize("cap,length", [(128, 1), (128, 65), (640, 333)])
+def test_builds_for_many_rows(dev, orc, dh, B, cap, length):
+    """The builds for many rows against the split rows of few, bit for bit, and the oracle: one position, a chunk's last few, two chunks."""
+    heads, scale = 16, 1.0 / np.sqrt(dh)
+    k, v, q = (orc.round_bf16(orc.normal((B, n, heads, dh), 31 + i)) for i, n in enumerate((length, length, 1)))
+
+    def run(rows):
+        cache = Cache(dev, len(rows), heads, dh, cap, 16, shuffle_seed=4)
+        cache.append(k[rows].reshape(len(rows), length, -1), v[rows].reshape(len(rows), length, -1), length)
+        cache.advance(length - 1)
+        out = cache.attend(q[rows].reshape(len(rows), 1, -1), 1, scale)
+        cache.close()
+        return out
+
+    big = run(list(range(B)))
+    for rows in ([0, 1], [B - 1]):
+        assert np.array_equal(run(rows), big[rows])
+    got = big.reshape(B, heads, dh)
+    for b, h in ((0, 0), (B - 1, 15)):
+        exp = orc.attention_slice(orc.widen_bf16(q[b, :, h]), orc.widen_bf16(k[b, :, h]), orc.widen_bf16(v[b, :, h]), length - 1, scale)
+        assert orc.close(orc.bf16_round_trip(exp), orc.widen_bf16(got[b, h][None]), TOL)

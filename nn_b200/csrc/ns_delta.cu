@@ -69,6 +69,14 @@ NS_DEVINL void conv_load(const NsSource& s, int64_t idx, float (&x)[V])
     }
 }
 
+// CTAs an SM that a build is held to; left to itself the compiler spills for more.
+__host__ __device__ constexpr int conv_ctas(int v, int taps, int piece, int src)
+{
+    if (taps > 4 || v == 1) return 1;
+    if (v == 2) return piece == 1 ? 8 : 6;
+    return piece == 1 ? (src == CONV_SLABS ? 5 : 6) : (src == CONV_SLABS ? 3 : 4);
+}
+
 // The sums of v[0..8) over the warp, in the order ns_warp_sum takes: lane l has that of v[l / 4].
 NS_DEVINL float conv_sum8(float (&v)[8], int lane)
 {
@@ -92,7 +100,7 @@ NS_DEVINL float conv_sum8(float (&v)[8], int lane)
 // channels, bf16 in, float out 112 -> 67 (floor 31), of 6144 157 -> 99; one token of 64 sequences, 6144 channels of 3 slabs 10.5 -> 5.2, of 250
 // sequences, 4096 channels of 4 slabs 19.8 -> 10.3; 4 x 100 of 2 slabs 13.4 -> 10.8.  Eight pieces a warp instead of four: 66, 96, but 3 x 300 tokens 28 for 16.
 template <typename T, int V, int TAPS, int PIECE, int SRC>
-__global__ void __launch_bounds__(128) ns_short_conv_slide_kernel(const ConvArgs a, int span, int units, int pieces)
+__global__ void __launch_bounds__(128, conv_ctas(V, TAPS, PIECE, SRC)) ns_short_conv_slide_kernel(const ConvArgs a, int span, int units, int pieces)
 {
     ns_pdl_wait();
     ns_pdl_trigger();

@@ -11,7 +11,9 @@
 // The recurrence is a 32-bit one, so each product's operands are split into two bf16 halves (x = hi + lo, 16 mantissa bits) and
 // multiplied as hi hi + hi lo + lo hi into 32-bit accumulators; the state stays in 32-bit registers from chunk to chunk.
 //
-// One CTA of 8 warps walks the chunks of one (sequence, head, up to 128 value columns).
+// One CTA of 8 warps walks the chunks of one (sequence, head, up to 128 value columns).  What bounds it is the chain of a chunk's phases, a third of it
+// mma.sync: 16 sequences x 16 heads of 128, 512 tokens, decays per head 361 us (40 000 cycles a chunk), per channel 626 -> 532 us (74 000 ->
+// 62 000) with the decay projection loaded at once, the diagonal blocks' rows dealt evenly to the warps, and keys read back from shared memory.
 #include "ns_mma.cuh"
 #include "ns_seq.cuh"
 
@@ -167,7 +169,13 @@ __global__ void __launch_bounds__(256, 1) ns_delta_chunk_kernel(const ChunkArgs 
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(qh + (row0 + CH + r) * a.q_ld + c));
                 }
                 if (v0 + c < vdim && c < DV) asm volatile("prefetch.global.L2 [%0];" ::"l"(vh + (row0 + CH + r) * a.v_ld + c));
+                if (CHANNEL && a.a.splits == 1 && c < dim)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const float*>(a.a.ptr) + (row0 + CH + r) * a.a.ld + a.a_col + head * dim + c));
             }
+        }
+        if (c0 + CH + tid < a.steps && tid < CH) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const float*>(a.b.ptr) + (row0 + CH + tid) * a.b.ld + a.b_col + head));
+            if (!CHANNEL) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const float*>(a.a.ptr) + (row0 + CH + tid) * a.a.ld + a.a_col + head));
         }
         constexpr int QUADS = DK / 4;      // a thread takes four channels of a row
         // keys and queries of elements e0, e0 + stride, ... (four of them), all loaded before the caller stores any
@@ -183,21 +191,38 @@ __global__ void __launch_bounds__(256, 1) ns_delta_chunk_kernel(const ChunkArgs 
             }
         };
         // ------------------------------------------------------------ step sizes, running decays (slabs in turn: together they spilled)
-        if (tid < CH) sBeta[tid] = tid < n ? ns_sigmoid(ns_source_at<NS_IN_TURN>(a.b, (row0 + tid) * a.b.ld + a.b_col + head)) : 0.0f;
+        const float step = tid < n ? ns_source_at<NS_IN_TURN>(a.b, (row0 + tid) * a.b.ld + a.b_col + head) : 0.0f;   // (n <= CH)
         if (CHANNEL) {
-            const int c = (tid % QUADS) * 4;
+            int th = tid;                                                        // (addresses made from it are not kept from chunk to chunk)
+            asm volatile("" : "+r"(th));
+            const int c = (th % QUADS) * 4;
             const float4 dt = row4(a.dt_bias + (int64_t)head * dim, c, dim);
-#pragma unroll 8
-            for (int t = tid / QUADS; t < CH; t += 256 / QUADS) {
-                float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (t < n && c < dim) {
-                    const int64_t at = (row0 + t) * a.a.ld + a.a_col + head * dim + c;
-                    x = ns_source_at4<NS_IN_TURN>(a.a, at);
-                    x = make_float4(fmaxf(-rate2 * softplus(x.x + dt.x), WEAKEST), fmaxf(-rate2 * softplus(x.y + dt.y), WEAKEST),
-                                    fmaxf(-rate2 * softplus(x.z + dt.z), WEAKEST), fmaxf(-rate2 * softplus(x.w + dt.w), WEAKEST));
-                }
-                *reinterpret_cast<float4*>(sG + t * L::LG + c) = x;
+            // a thread's tokens; all loads of a finished matrix before the first is used (one after the other they were 10 000 of a chunk's 74 000 cycles)
+            constexpr int PASSES = CH * QUADS / 256;
+            float4 x[PASSES];
+#pragma unroll
+            for (int i = 0; i < PASSES; i++) {
+                const int t = th / QUADS + i * (256 / QUADS);
+                x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (a.a.splits == 1 && t < n && c < dim)
+                    x[i] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.a.ptr) + (row0 + t) * a.a.ld + a.a_col + head * dim + c);
             }
+            if (a.a.splits != 1) {
+#pragma unroll
+                for (int i = 0; i < PASSES; i++) {
+                    const int t = th / QUADS + i * (256 / QUADS);
+                    if (t < n && c < dim) x[i] = ns_source_at4<NS_IN_TURN>(a.a, (row0 + t) * a.a.ld + a.a_col + head * dim + c);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < PASSES; i++) {
+                const int t = th / QUADS + i * (256 / QUADS);
+                if (t < n && c < dim)
+                    x[i] = make_float4(fmaxf(-rate2 * softplus(x[i].x + dt.x), WEAKEST), fmaxf(-rate2 * softplus(x[i].y + dt.y), WEAKEST),
+                                       fmaxf(-rate2 * softplus(x[i].z + dt.z), WEAKEST), fmaxf(-rate2 * softplus(x[i].w + dt.w), WEAKEST));
+                *reinterpret_cast<float4*>(sG + t * L::LG + c) = x[i];
+            }
+            if (tid < CH) sBeta[tid] = tid < n ? ns_sigmoid(step) : 0.0f;
             __syncthreads();
             if (tid < DK) {
                 float s = 0.0f;
@@ -222,6 +247,7 @@ __global__ void __launch_bounds__(256, 1) ns_delta_chunk_kernel(const ChunkArgs 
             sGam[2 * lane] = s - x[1];
             sGam[2 * lane + 1] = s;
         }
+        if (!CHANNEL && tid < CH) sBeta[tid] = tid < n ? ns_sigmoid(step) : 0.0f;
         __syncthreads();
 
         // ------------------------------------------------------------ A and P
@@ -340,8 +366,9 @@ __global__ void __launch_bounds__(256, 1) ns_delta_chunk_kernel(const ChunkArgs 
             // the 16 x 16 blocks on the diagonal, pair by pair: 16 lanes share a row, each a sixteenth of the channels
             constexpr int CPL = DK / 16;
             const int hl = lane & 15;
-            for (int task = (warp + 2) & 7; task < CH / 2; task += 8) {
-                const int blk = task >> 3, ii = (lane >> 4) ? 15 - (task & 7) : (task & 7), i = blk * 16 + ii;
+            for (int blk = 0; blk < 4; blk++) {
+                // two neighbouring rows a warp, which end in the same group of columns; from block to block a warp's rows change sides, so all have as much
+                const int pair = (blk & 1) ? 7 - warp : warp, ii = 2 * pair + (lane >> 4), i = blk * 16 + ii;
                 const int ch = hl * 4;      // channels ch + 64 y: 16 lanes read 256 neighbouring bytes
                 float ki[CPL], qi[CPL], gi[CPL];
 #pragma unroll
@@ -354,7 +381,7 @@ __global__ void __launch_bounds__(256, 1) ns_delta_chunk_kernel(const ChunkArgs 
                     gi[x] = G.x; gi[x + 1] = G.y; gi[x + 2] = G.z; gi[x + 3] = G.w;
                 }
                 // columns in groups of four; what lies right of the diagonal is dropped afterwards
-                const int groups = (max(task & 7, 15 - (task & 7)) >> 2) + 1;
+                const int groups = (pair >> 1) + 1;
 #pragma unroll 1
                 for (int j0 = 0; j0 < groups * 4; j0 += 4) {
                     const int t0 = blk * 16 + j0;
@@ -415,18 +442,27 @@ __global__ void __launch_bounds__(256, 1) ns_delta_chunk_kernel(const ChunkArgs 
 #pragma unroll
             for (int i = 0; i < 16; i++) blk[i * L::LA + col] = x[i];
         } else if (CHANNEL) {
-            for (int e0 = tid - 64; e0 < CH * QUADS; e0 += 768) {
-                float4 k4[4], q4[4];
-                load_rows(e0, 192, k4, q4);
+            constexpr int BATCH = 3;                                             // queries on their way together; the keys are still in sK
+            int th = tid - 64;                                                   // (addresses made from it are not kept from chunk to chunk)
+            asm volatile("" : "+r"(th));
+            for (int e0 = th; e0 < CH * QUADS; e0 += BATCH * 192) {
+                float4 q4[BATCH];
 #pragma unroll
-                for (int x = 0; x < 4; x++) {
+                for (int x = 0; x < BATCH; x++) {
+                    const int e = e0 + 192 * x, t = e / QUADS, c = (e % QUADS) * 4;
+                    q4[x] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (t < n) q4[x] = row4(qh + (row0 + t) * a.q_ld, c, dim);
+                }
+#pragma unroll
+                for (int x = 0; x < BATCH; x++) {
                     const int e = e0 + 192 * x, t = e / QUADS, c = (e % QUADS) * 4;
                     if (e >= CH * QUADS) break;
+                    const float4 k4 = *reinterpret_cast<const float4*>(sK + t * L::LG + c);
                     const float4 G = *reinterpret_cast<const float4*>(sG + t * L::LG + c), f = exp2_of(G, make_float4(0.f, 0.f, 0.f, 0.f));
                     const uint32_t at = base + (t * L::LK + c) * 2;
-                    st_split4(at + L::KT, at + L::KT + L::KMAT, times(k4[x], f));
+                    st_split4(at + L::KT, at + L::KT + L::KMAT, times(k4, f));
                     st_split4(at + L::QT, at + L::QT + L::KMAT, times(q4[x], f));
-                    st_split4(at + L::KB, at + L::KB + L::KMAT, times(k4[x], exp2_of(*reinterpret_cast<const float4*>(sG + (CH - 1) * L::LG + c), G)));
+                    st_split4(at + L::KB, at + L::KB + L::KMAT, times(k4, exp2_of(*reinterpret_cast<const float4*>(sG + (CH - 1) * L::LG + c), G)));
                 }
             }
         }

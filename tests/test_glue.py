@@ -197,3 +197,21 @@ def test_embed_pos_of_bf16_tables(dev, orc, batch, steps, dim):
     at = np.minimum(p0 + np.arange(steps), ctx - 1)
     exp = orc.round_bf16(orc.widen_bf16(tok)[np.clip(ids, 0, V - 1)] + orc.widen_bf16(pos)[at][None])
     assert np.array_equal(y.download((batch, steps, dim)), exp)
+
+
+@pytest.mark.parametrize("rows", [1183, 1184, 1185, 2400])
+def test_quantize_many_float_rows_a_row_ahead(dev, orc, rows):
+    """Eight rows an SM and more: the CTAs walk the rows with the next one in registers.  The same bytes and scales as for few rows at a time,
+    rows with a NaN, an infinity, zeros or subnormal values among them."""
+    cols = 4096
+    x = orc.normal((rows, cols), 84, 1.5)
+    x[5, 7], x[6, 4095], x[7], x[8] = np.nan, np.inf, 0.0, 1e-41
+    dx, dq, ds, dq2, ds2 = dev.from_numpy(x), dev.empty(rows * cols, N.NS_I8), dev.empty(rows), dev.empty(rows * cols, N.NS_I8), dev.empty(rows)
+    N.call("ns_quantize_rows_i8", dev.handle, dx.ptr, N.NS_F32, C.c_int64(rows), cols, dq.ptr, ds.ptr)
+    for r0 in range(0, rows, 600):
+        N.call("ns_quantize_rows_i8", dev.handle, C.c_uint64(dx.ptr + r0 * cols * 4), N.NS_F32, C.c_int64(min(600, rows - r0)), cols, C.c_uint64(dq2.ptr + r0 * cols),
+               C.c_uint64(ds2.ptr + r0 * 4))
+    dev.synchronize()
+    assert np.array_equal(ds.download().view(np.uint32), ds2.download().view(np.uint32)) and np.array_equal(dq.download(), dq2.download())
+    q, s = orc.quantize_rows_i8(x[9:])
+    assert np.array_equal(s, ds.download()[9:]) and np.array_equal(q, dq.download((rows, cols))[9:])

@@ -61,6 +61,18 @@ __global__ void __launch_bounds__(128) ns_embed_ngram_kernel(const int32_t* __re
     }
 }
 
+// The RMS row kernels of few rows are launched while the product in front of them still runs: generating with 7 sequences (topidra), 64 tokens,
+// 15.5 -> 15.2 ms; with 64 (fabezen) level, so from nine rows on they wait, as the products in front then are other kernels.
+constexpr unsigned RMS_EARLY_ROWS = 8;
+// Their vectors towards L2, before the wait: a hint, nothing is read.
+NS_DEVINL void rms_prefetch(const float* v, const float* w, int cols)
+{
+    for (int c = threadIdx.x * 32; c < cols; c += blockDim.x * 32) {
+        if (v != nullptr) asm volatile("prefetch.global.L2 [%0];" ::"l"(v + c));
+        if (w != nullptr) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + c));
+    }
+}
+
 // ---------------------------------------------------------------------------------------------
 // x_out = x + alpha * source; y = x_out / sqrt(mean(x_out^2) + eps) * w
 // ---------------------------------------------------------------------------------------------
@@ -83,10 +95,10 @@ __global__ void __launch_bounds__(256) ns_rms_rows_kernel(const RmsArgs a)
     extern __shared__ float4 rms_row4[];
     float* buf = reinterpret_cast<float*>(rms_row4);
     __shared__ float red[8];
-    ns_pdl_wait();
     // asked for now, read after the reduction (see ns_rms_post_rows_vec_kernel)
-    if (VEC && SLABS != NS_ONE_SLAB && a.w != nullptr)
-        for (int c = threadIdx.x * 32; c < a.cols; c += blockDim.x * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.w + c));
+    if (VEC && (SLABS != NS_ONE_SLAB || gridDim.x <= RMS_EARLY_ROWS)) rms_prefetch(nullptr, a.w, a.cols);
+    ns_pdl_wait();
+    const float* norm_w = ns_after_wait(a.w);
     const int row = a.row_map != nullptr ? a.row_map[blockIdx.x] : (int)blockIdx.x;
     const int64_t base = (int64_t)row * a.cols;
     float ss = 0.0f;
@@ -118,11 +130,11 @@ __global__ void __launch_bounds__(256) ns_rms_rows_kernel(const RmsArgs a)
     if (VEC) {
         for (int c = threadIdx.x * 4; c < a.cols; c += blockDim.x * 4) {
             const float4 v = *reinterpret_cast<const float4*>(buf + c);
-            const float4 w = __ldg(reinterpret_cast<const float4*>(a.w + c));
+            const float4 w = __ldg(reinterpret_cast<const float4*>(norm_w + c));
             ns_store4(y + c, make_float4(v.x * inv * w.x, v.y * inv * w.y, v.z * inv * w.z, v.w * inv * w.w));
         }
     } else {
-        for (int c = threadIdx.x; c < a.cols; c += blockDim.x) ns_store(y + c, buf[c] * inv * a.w[c]);
+        for (int c = threadIdx.x; c < a.cols; c += blockDim.x) ns_store(y + c, buf[c] * inv * norm_w[c]);
     }
     for (int c = a.cols + threadIdx.x; c < a.y_ld; c += blockDim.x) ns_store(y + c, 0.0f);
 }
@@ -143,7 +155,9 @@ __global__ void __launch_bounds__(256) ns_rms_post_rows_vec_kernel(const PostRms
     constexpr bool EARLY = SLABS != NS_ONE_SLAB && Q <= 2;
     const RmsArgs& a = p.r;
     __shared__ float red[2][8];
+    if (SLABS != NS_ONE_SLAB || gridDim.x <= RMS_EARLY_ROWS) rms_prefetch(p.post_w, a.w, a.cols);
     ns_pdl_wait();
+    const float *post_w = ns_after_wait(p.post_w), *norm_w = ns_after_wait(a.w);
     const int row = blockIdx.x;
     const int64_t base = (int64_t)row * a.cols;
     float4 s[Q], x[Q], pw[EARLY ? Q : 1], nw[EARLY ? Q : 1];
@@ -155,8 +169,8 @@ __global__ void __launch_bounds__(256) ns_rms_post_rows_vec_kernel(const PostRms
         for (int i = 0; i < Q; i++) {
             const int c = (threadIdx.x + 256 * i) * 4;
             if (c >= a.cols) continue;
-            pw[i] = __ldg(reinterpret_cast<const float4*>(p.post_w + c));
-            if (a.w != nullptr) nw[i] = __ldg(reinterpret_cast<const float4*>(a.w + c));
+            pw[i] = __ldg(reinterpret_cast<const float4*>(post_w + c));
+            if (a.w != nullptr) nw[i] = __ldg(reinterpret_cast<const float4*>(norm_w + c));
         }
     }
 #pragma unroll
@@ -182,7 +196,7 @@ __global__ void __launch_bounds__(256) ns_rms_post_rows_vec_kernel(const PostRms
     for (int i = 0; i < Q; i++) {
         const int c = (threadIdx.x + 256 * i) * 4;
         if (c >= a.cols) continue;
-        const float4 w = EARLY ? pw[EARLY ? i : 0] : __ldg(reinterpret_cast<const float4*>(p.post_w + c));
+        const float4 w = EARLY ? pw[EARLY ? i : 0] : __ldg(reinterpret_cast<const float4*>(post_w + c));
         x[i] = make_float4(fmaf(s[i].x * post, w.x, x[i].x), fmaf(s[i].y * post, w.y, x[i].y), fmaf(s[i].z * post, w.z, x[i].z), fmaf(s[i].w * post, w.w, x[i].w));
         *reinterpret_cast<float4*>(a.x_out + base + c) = x[i];
         ss = fmaf(x[i].x, x[i].x, ss); ss = fmaf(x[i].y, x[i].y, ss); ss = fmaf(x[i].z, x[i].z, ss); ss = fmaf(x[i].w, x[i].w, ss);
@@ -194,7 +208,7 @@ __global__ void __launch_bounds__(256) ns_rms_post_rows_vec_kernel(const PostRms
     for (int i = 0; i < Q; i++) {
         const int c = (threadIdx.x + 256 * i) * 4;
         if (c >= a.cols) continue;
-        const float4 w = EARLY ? nw[EARLY ? i : 0] : __ldg(reinterpret_cast<const float4*>(a.w + c));
+        const float4 w = EARLY ? nw[EARLY ? i : 0] : __ldg(reinterpret_cast<const float4*>(norm_w + c));
         ns_store4(y + c, make_float4(x[i].x * inv * w.x, x[i].y * inv * w.y, x[i].z * inv * w.z, x[i].w * inv * w.w));
     }
     for (int c = a.cols + threadIdx.x; c < a.y_ld; c += blockDim.x) ns_store(y + c, 0.0f);
@@ -403,7 +417,8 @@ extern "C" int ns_rms_rows(ns_device_t h, uint64_t x, uint64_t src, int splits, 
     const size_t smem = (size_t)((cols + 3) & ~3) * 4;
     auto launch = [&](auto kernel) -> int {
         if (smem > 48 * 1024) NS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        NS_CUDA(ns_launch_plain(kernel, dim3((unsigned)rows), dim3(256), smem, d->stream, a));
+        if (rows <= RMS_EARLY_ROWS) NS_CUDA(ns_launch_pdl(kernel, dim3((unsigned)rows), dim3(256), smem, d->stream, a));
+        else NS_CUDA(ns_launch_plain(kernel, dim3((unsigned)rows), dim3(256), smem, d->stream, a));
         return NS_OK;
     };
     // 64 x 2047 of 8 slabs: 6.2 us together, 8.7 in turn; 8192 x 2047 of one slab: 83 in the build for many, 62 in its own
@@ -440,7 +455,8 @@ extern "C" int ns_rms_post_rows(ns_device_t h, uint64_t x, uint64_t src, int spl
     const size_t smem = vec ? 0 : (size_t)((cols + 3) & ~3) * 4;
     auto launch = [&](auto kernel) -> int {
         if (smem > 48 * 1024) NS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        NS_CUDA(ns_launch_plain(kernel, dim3((unsigned)rows), dim3(256), smem, d->stream, p));
+        if (rows <= RMS_EARLY_ROWS) NS_CUDA(ns_launch_pdl(kernel, dim3((unsigned)rows), dim3(256), smem, d->stream, p));
+        else NS_CUDA(ns_launch_plain(kernel, dim3((unsigned)rows), dim3(256), smem, d->stream, p));
         return NS_OK;
     };
     auto pick = [&](auto zero) -> int {

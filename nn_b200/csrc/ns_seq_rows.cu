@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(128) ns_embed_ngram_kernel(const int32_t* __re
 }
 
 // The RMS row kernels of few rows are launched while the product in front of them still runs: generating with 7 sequences (topidra), 64 tokens,
-// 15.5 -> 15.2 ms; with 64 (fabezen) level, so from nine rows on they wait, as the products in front then are other kernels.
+// 15.5 -> 15.0 ms (seven rows of 2048 with both norms in a chain of their own 3.2 -> 2.3 us); with 64 (fabezen) level, so from nine rows on they wait, as the products in front then are other kernels.
 constexpr unsigned RMS_EARLY_ROWS = 8;
 // Their vectors towards L2, before the wait: a hint, nothing is read.
 NS_DEVINL void rms_prefetch(const float* v, const float* w, int cols)
@@ -96,9 +96,9 @@ __global__ void __launch_bounds__(256) ns_rms_rows_kernel(const RmsArgs a)
     float* buf = reinterpret_cast<float*>(rms_row4);
     __shared__ float red[8];
     // asked for now, read after the reduction (see ns_rms_post_rows_vec_kernel)
-    if (VEC && (SLABS != NS_ONE_SLAB || gridDim.x <= RMS_EARLY_ROWS)) rms_prefetch(nullptr, a.w, a.cols);
+    if (VEC && SLABS != NS_ONE_SLAB) rms_prefetch(nullptr, a.w, a.cols);
     ns_pdl_wait();
-    const float* norm_w = ns_after_wait(a.w);
+    const float* norm_w = SLABS != NS_ONE_SLAB ? ns_after_wait(a.w) : a.w;
     const int row = a.row_map != nullptr ? a.row_map[blockIdx.x] : (int)blockIdx.x;
     const int64_t base = (int64_t)row * a.cols;
     float ss = 0.0f;
@@ -155,9 +155,10 @@ __global__ void __launch_bounds__(256) ns_rms_post_rows_vec_kernel(const PostRms
     constexpr bool EARLY = SLABS != NS_ONE_SLAB && Q <= 2;
     const RmsArgs& a = p.r;
     __shared__ float red[2][8];
-    if (SLABS != NS_ONE_SLAB || gridDim.x <= RMS_EARLY_ROWS) rms_prefetch(p.post_w, a.w, a.cols);
+    // (the build for one slab is never launched early, and left to schedule these loads as it likes)
+    if (SLABS != NS_ONE_SLAB) rms_prefetch(p.post_w, a.w, a.cols);
     ns_pdl_wait();
-    const float *post_w = ns_after_wait(p.post_w), *norm_w = ns_after_wait(a.w);
+    const float *post_w = SLABS != NS_ONE_SLAB ? ns_after_wait(p.post_w) : p.post_w, *norm_w = SLABS != NS_ONE_SLAB ? ns_after_wait(a.w) : a.w;
     const int row = blockIdx.x;
     const int64_t base = (int64_t)row * a.cols;
     float4 s[Q], x[Q], pw[EARLY ? Q : 1], nw[EARLY ? Q : 1];
@@ -422,7 +423,7 @@ extern "C" int ns_rms_rows(ns_device_t h, uint64_t x, uint64_t src, int splits, 
         return NS_OK;
     };
     // 64 x 2047 of 8 slabs: 6.2 us together, 8.7 in turn; 8192 x 2047 of one slab: 83 in the build for many, 62 in its own
-    return ns_pick_slabs<NS_ONE_SLAB>(a.src.splits > 1, [&](auto slabs) {
+    return ns_pick_slabs<NS_ONE_SLAB>(a.src.splits > 1 || rows <= RMS_EARLY_ROWS, [&](auto slabs) {
         constexpr int S = decltype(slabs)::value;
         if (w == 0 || out_dtype == NS_F32) return vec ? launch(ns_rms_rows_kernel<float, true, S>) : launch(ns_rms_rows_kernel<float, false, S>);
         return vec ? launch(ns_rms_rows_kernel<uint16_t, true, S>) : launch(ns_rms_rows_kernel<uint16_t, false, S>);
@@ -461,7 +462,7 @@ extern "C" int ns_rms_post_rows(ns_device_t h, uint64_t x, uint64_t src, int spl
     };
     auto pick = [&](auto zero) -> int {
         using T = decltype(zero);
-        return ns_pick_slabs<NS_ONE_SLAB>(a.src.splits > 1, [&](auto slabs) {
+        return ns_pick_slabs<NS_ONE_SLAB>(a.src.splits > 1 || rows <= RMS_EARLY_ROWS, [&](auto slabs) {
             constexpr int S = decltype(slabs)::value;
             if (!vec) return launch(ns_rms_post_rows_kernel<T, S>);
             if (cols <= 1024) return launch(ns_rms_post_rows_vec_kernel<T, 1, S>);

@@ -62,7 +62,8 @@ __global__ void __launch_bounds__(128) ns_embed_ngram_kernel(const int32_t* __re
 }
 
 // The RMS row kernels of few rows are launched while the product in front of them still runs: generating with 7 sequences (topidra), 64 tokens,
-// 15.5 -> 15.0 ms (seven rows of 2048 with both norms in a chain of their own 3.2 -> 2.3 us); with 64 (fabezen) level, so from nine rows on they wait, as the products in front then are other kernels.
+// 15.5 -> 15.0 ms (seven rows of 2048 with both norms, in a chain of their own, 3.2 -> 2.3 us); with 64 (fabezen) level, so from nine rows
+// on they wait, as the products in front then are other kernels.
 constexpr unsigned RMS_EARLY_ROWS = 8;
 // Their vectors towards L2, before the wait: a hint, nothing is read.
 NS_DEVINL void rms_prefetch(const float* v, const float* w, int cols)

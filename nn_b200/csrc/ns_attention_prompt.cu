@@ -507,6 +507,13 @@ __global__ void __launch_bounds__(PA_THREADS, 1) ns_attention_prompt_kernel(cons
                 pa_exponentials<0>(s, p.scale_log2, neg_m, sum, pk);
                 hand_over(0, pk);
                 pa_exponentials<64>(s, p.scale_log2, neg_m, sum, pk);
+                // A wait names a phase by its parity, so O_DONE may be asked neither two phases early nor one late.  With SOLO the last scores come before the
+                // P.V of the block in front, which may still wait for another warp's P or for its V: that P.V is waited for here, before this block's own
+                // can end, and the read-out then waits for the phase that follows.
+                if (SOLO && j > 0 && j + 1 == n) {
+                    ok = wait(PB_O_DONE + g, k - 1, 12);
+                    if (!ok) break;
+                }
                 hand_over(1, pk);
                 float l0, l1;
                 pa_split(pa_add2(sum[0], sum[1]), l0, l1);

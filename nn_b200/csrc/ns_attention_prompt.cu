@@ -81,10 +81,17 @@ __device__ __forceinline__ float pa_exp2(float x)
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// maxima of which a NaN is one
 __device__ __forceinline__ float pa_max3(float a, float b, float c)
 {
     float y;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    return y;
+}
+__device__ __forceinline__ float pa_max2(float a, float b)
+{
+    float y;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
     return y;
 }
 __device__ __forceinline__ uint64_t pa_pair(float lo, float hi)
@@ -107,7 +114,7 @@ __device__ __forceinline__ uint64_t pa_fma2(uint64_t a, uint64_t b, uint64_t c)
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(y) : "l"(a), "l"(b), "l"(c));
     return y;
 }
-// The maximum of a row's scores.
+// The maximum of a row's scores; NaN where one of them is.
 __device__ __forceinline__ float pa_row_max(const float (&s)[PA_KB])
 {
     float m[8];
@@ -118,13 +125,13 @@ __device__ __forceinline__ float pa_row_max(const float (&s)[PA_KB])
 #pragma unroll
         for (int q = 0; q < 8; q++) m[q] = pa_max3(m[q], s[c + 2 * q], s[c + 2 * q + 1]);
 #pragma unroll
-    for (int q = 0; q < 8; q++) m[q] = fmaxf(m[q], s[PA_KB - 8 + q]);
-    return pa_max3(pa_max3(m[0], m[1], m[2]), pa_max3(m[3], m[4], m[5]), fmaxf(m[6], m[7]));
+    for (int q = 0; q < 8; q++) m[q] = pa_max2(m[q], s[PA_KB - 8 + q]);
+    return pa_max3(pa_max3(m[0], m[1], m[2]), pa_max3(m[3], m[4], m[5]), pa_max2(m[6], m[7]));
 }
 
 // 2^x of two values on the multiply-add pipe, x <= 126: x = n + f with f in [-1/2, 1/2], 2^f as the polynomial of degree 5 with the
 // least relative error under p(0) = 1 (a linear programme over 4001 points of the interval; 2^-22.5 with float rounding, ex2.approx
-// states 2^-22), n added to the exponent.  x at or below -127 (a masked score) gives 0.
+// states 2^-22), n added to the exponent.  x at or below -127 (a masked score) gives 0, and so does a NaN: see neg_m.
 __device__ __forceinline__ void pa_exp2_pair(uint64_t x, float& y0, float& y1)
 {
     float x0, x1;
@@ -471,7 +478,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1) ns_attention_prompt_kernel(cons
                 const float mx = pa_row_max(s);
                 float alpha = 1.0f;
                 bool rescale = false;
-                if (mx != -INFINITY && (m_ref == -INFINITY || (mx - m_ref) * p.scale_log2 > (j < PA_EARLY ? 0.0f : 8.0f))) {
+                if (mx != -INFINITY && (m_ref == -INFINITY || !((mx - m_ref) * p.scale_log2 <= (j < PA_EARLY ? 0.0f : 8.0f)))) {
                     alpha = m_ref == -INFINITY ? 0.0f : pa_exp2((m_ref - mx) * p.scale_log2);
                     rescale = m_ref != -INFINITY;
                     m_ref = mx;
@@ -493,7 +500,9 @@ __global__ void __launch_bounds__(PA_THREADS, 1) ns_attention_prompt_kernel(cons
                         ns_tmem_st32(o_addr + c * 32, ob);
                     }
                 }
-                const float neg_m = m_ref == -INFINITY ? 0.0f : -m_ref * p.scale_log2;
+                // A score of NaN or +infinity makes a row NaN, whichever key's it is.  Both show in the maximum, which then makes every weight of
+                // the row NaN (0 m_ref is NaN, else nothing); keeping them through the polynomial cost 1 to 4 % of a launch.
+                const float neg_m = m_ref == -INFINITY ? 0.0f : fmaf(m_ref, 0.0f, -m_ref * p.scale_log2);
                 uint64_t sum[2] = {0, 0};
                 auto hand_over = [&](int hf, const uint32_t (&pk)[32]) {
                     __syncwarp();

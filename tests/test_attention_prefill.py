@@ -143,3 +143,46 @@ def test_tiles_of_one_group_and_of_two(dev, orc, S, causal):
         exp = orc.attention_slice(*(orc.widen_bf16(x[0, h]) for x in (q, k, v)), 0, scale, causal)
         got = orc.widen_bf16(one[0, h])
         assert orc.close(orc.bf16_round_trip(exp), got, TOL), (h, orc.max_err(exp, got))
+
+
+@pytest.mark.parametrize("S,batch", [(300, 1), (300, 100)])      # tiles of one group, of two
+@pytest.mark.parametrize("causal", [True, False])
+def test_scores_that_are_no_numbers(dev, S, batch, causal):
+    """A NaN in a key makes every row that sees it NaN, whichever key it is (one exponential in eight is a polynomial); so does a score of +infinity.  A score of
+    -infinity weighs nothing.  Other rows keep their bits."""
+    rng = np.random.default_rng(9)
+    heads, scale = 2, 0.1
+    q, k, v = (rng.standard_normal((heads, S, DH)).astype(np.float32) for _ in range(3))
+    q[:, ::2, 0], q[:, 1::2, 0] = 1, -1
+    bits = lambda a: (np.ascontiguousarray(a, np.float32).view(np.uint32) >> 16).astype(np.uint16)
+    wide = lambda b: (b.astype(np.uint32) << 16).view(np.float32).astype(np.float64)
+
+    def run(key):
+        many = [np.repeat(bits(x)[None], batch, 0) for x in (q, key, v)]
+        out = _run_bhsd(dev, *many, batch, heads, S, scale, causal)
+        assert np.array_equal(out, np.repeat(out[:1], batch, 0))
+        return out[0]
+
+    clean = run(k)
+    rows = np.arange(S)
+    for j in [*range(16), 62, 63, 127, 128, 142, 143, 255, 256, 270, 298, 299]:
+        sees = rows >= j if causal else rows >= 0
+        for value in (np.nan, np.inf):
+            key = k.copy()
+            key[:, j, 0] = value
+            got = run(key)
+            lost = sees & (np.isnan(value) | (rows % 2 == 0))
+            assert np.isnan(wide(got[:, lost])).all(), (j, value)
+            assert np.array_equal(got[:, ~sees], clean[:, ~sees]), (j, value)
+            rest = np.nonzero(sees & ~lost)[0][:: 7]
+            if len(rest):
+                for h in range(heads):
+                    s = wide(bits(q[h, rest])) @ wide(bits(k[h])).T * scale
+                    s[:, j] = -np.inf
+                    if causal:
+                        s[rows[None, :] > rest[:, None]] = -np.inf
+                    p = np.exp(s - s.max(1, keepdims=True))
+                    p /= p.sum(1, keepdims=True)
+                    value_rows = wide(bits(v[h]))
+                    # weights and results are rounded to bf16, whose numbers are 2^-7 apart: 2^-8 of each term, and of the sum
+                    assert np.all(np.abs(wide(got[h, rest]) - p @ value_rows) <= 2.0 ** -7 * (p @ np.abs(value_rows)))

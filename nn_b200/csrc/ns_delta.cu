@@ -69,12 +69,15 @@ NS_DEVINL void conv_load(const NsSource& s, int64_t idx, float (&x)[V])
     }
 }
 
-// CTAs an SM that a build is held to; left to itself the compiler spills for more.
+// CTAs an SM that a build is held to (no build spills more than 8 bytes).  Without a bound the builds for one and two tokens take registers that cost them CTAs
+// where there are many sequences: 250 of 32 heads of 32 channels 7.0 us against 5.0, heads of 64 with six taps 13.7 against 9.2; the build for prompts with six taps
+// and heads of 128 took 178 registers, two CTAs an SM, 16 x 512 tokens of bf16 227 us against 170.
 __host__ __device__ constexpr int conv_ctas(int v, int taps, int piece, int src)
 {
-    if (taps > 4 || v == 1) return 1;
-    if (v == 2) return piece == 1 ? 8 : 6;
-    return piece == 1 ? (src == CONV_SLABS ? 5 : 6) : (src == CONV_SLABS ? 3 : 4);
+    if (v == 1) return piece == 8 ? 1 : (taps > 4 || src == CONV_SLABS ? 7 : 8);
+    if (taps > 4) return v == 4 ? (piece == 8 && src != CONV_SLABS ? 3 : 1) : (piece < 8 ? 5 : 1);
+    if (v == 2) return piece < 8 ? 8 : 6;
+    return piece < 8 ? (src == CONV_SLABS ? 5 : 6) : (src == CONV_SLABS ? 3 : 4);
 }
 
 // The sums of v[0..8) over the warp, in the order ns_warp_sum takes: lane l has that of v[l / 4].
@@ -93,7 +96,7 @@ NS_DEVINL float conv_sum8(float (&v)[8], int lane)
     return r + __shfl_xor_sync(0xffffffffu, r, 1);
 }
 
-// PIECE: tokens whose inputs are in registers together (8; 1 for a step of one token, whose loads are then all there is).  What bounds a prompt is
+// PIECE: tokens whose inputs are in registers together: 8, or all of a step of one or two (whose loads are then all there is).  What bounds a prompt is
 // the arithmetic of a warp, not HBM: the tokens of a piece are computed side by side in place of their inputs, last one first, and the heads' lengths
 // of all eight are summed in one butterfly, so that a lane takes one root and one division where it took eight.
 // Weights of four taps come as one load a channel, and a bf16 matrix a piece ahead.  Against one token after the other (us): 16 x 512 tokens of 4096
@@ -116,20 +119,27 @@ __global__ void __launch_bounds__(128, conv_ctas(V, TAPS, PIECE, SRC)) ns_short_
     float* hist = g.hist + (int64_t)slot * a.hist_slot_stride + ch;
     const int64_t src0 = (int64_t)b * a.steps * a.src.ld + g.col + ch;
     const int per = CONV_WARP * pieces;
-    const int t0 = (span == 4 ? (int)blockIdx.x * 4 + warp : (int)blockIdx.x) * per, t1 = min(t0 + per, a.steps);
+    // (PIECE 1 and 2: all of a step's tokens)
+    const int t0 = PIECE < 8 ? 0 : (span == 4 ? (int)blockIdx.x * 4 + warp : (int)blockIdx.x) * per, t1 = PIECE < 8 ? PIECE : min(t0 + per, a.steps);
     float w[TAPS][V], back[TAPS][V];   // w[n]: weight of the input n tokens back; back[n]: the input n tokens before the piece
     const bool vec_w = TAPS == 4 && taps == 4 && (reinterpret_cast<uintptr_t>(g.w) & 15) == 0;
+    if (vec_w) {
 #pragma unroll
-    for (int i = 0; i < V; i++) {
-        float4 wi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (vec_w && mine) wi = __ldg(reinterpret_cast<const float4*>(g.w) + ch + i);
+        for (int i = 0; i < V; i++) {
+            const float4 wi = mine ? __ldg(reinterpret_cast<const float4*>(g.w) + ch + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-        for (int n = 0; n < TAPS; n++) {
-            back[n][i] = 0.0f;
-            if (vec_w) w[n][i] = n == 0 ? wi.w : (n == 1 ? wi.z : (n == 2 ? wi.y : wi.x));
-            else w[n][i] = mine && n < taps ? __ldg(g.w + (int64_t)(ch + i) * taps + taps - 1 - n) : 0.0f;
+            for (int n = 0; n < TAPS; n++) w[n][i] = n == 0 ? wi.w : (n == 1 ? wi.z : (n == 2 ? wi.y : wi.x));
         }
+    } else {
+#pragma unroll
+        for (int n = 0; n < TAPS; n++)
+#pragma unroll
+            for (int i = 0; i < V; i++) w[n][i] = mine && n < taps ? __ldg(g.w + (int64_t)(ch + i) * taps + taps - 1 - n) : 0.0f;
     }
+#pragma unroll
+    for (int n = 0; n < TAPS; n++)
+#pragma unroll
+        for (int i = 0; i < V; i++) back[n][i] = 0.0f;
     // the inputs of a piece: for one bf16 matrix they are asked for a piece ahead, as they lie in memory
     constexpr bool AHEAD = SRC == CONV_BF16 && V == 4;
     uint2 next[AHEAD ? PIECE : 1];
@@ -159,32 +169,56 @@ __global__ void __launch_bounds__(128, conv_ctas(V, TAPS, PIECE, SRC)) ns_short_
         // all inputs of a piece are on their way before the first is used
         float in[PIECE][V], ss[PIECE], last[TAPS][V];
 #pragma unroll
-        for (int j = 0; j < PIECE; j++) {
+        for (int j = 0; j < PIECE; j++)
 #pragma unroll
             for (int i = 0; i < V; i++) in[j][i] = 0.0f;
-            if constexpr (AHEAD) {
+        if constexpr (AHEAD) {
+#pragma unroll
+            for (int j = 0; j < PIECE; j++) {
                 in[j][0] = __uint_as_float(next[j].x << 16); in[j][1] = __uint_as_float(next[j].x & 0xFFFF0000u);
                 in[j][2] = __uint_as_float(next[j].y << 16); in[j][3] = __uint_as_float(next[j].y & 0xFFFF0000u);
-            } else if (mine && tp + j < t1) conv_load<V, SRC>(a.src, src0 + (int64_t)(tp + j) * a.src.ld, in[j]);
+            }
+            if (tp + PIECE < t1) ask(tp + PIECE);
+        } else if (V < 4 && SRC == CONV_ANY && a.src.dtype == NS_BF16) {
+            // widened after all of them are asked for (one by one each load was waited for: 16 x 512 tokens of 32 heads of 64 80 us, now 51)
+            uint32_t raw[PIECE][V];
+#pragma unroll
+            for (int j = 0; j < PIECE; j++)
+#pragma unroll
+                for (int i = 0; i < V; i++)
+                    raw[j][i] = mine && tp + j < t1 ? reinterpret_cast<const uint16_t*>(a.src.ptr)[src0 + (int64_t)(tp + j) * a.src.ld + i] : 0u;
+#pragma unroll
+            for (int j = 0; j < PIECE; j++)
+#pragma unroll
+                for (int i = 0; i < V; i++) in[j][i] = __uint_as_float(raw[j][i] << 16);
+        } else {
+#pragma unroll
+            for (int j = 0; j < PIECE; j++)
+                if (mine && tp + j < t1) conv_load<V, SRC>(a.src, src0 + (int64_t)(tp + j) * a.src.ld, in[j]);
         }
-        if (tp + PIECE < t1) ask(tp + PIECE);
         auto input = [&](int j, int i) { return j >= 0 ? in[j < 0 ? 0 : j][i] : back[j < 0 ? -j : 0][i]; };
 #pragma unroll
         for (int n = 1; n < TAPS; n++)
 #pragma unroll
             for (int i = 0; i < V; i++) last[n][i] = input(PIECE - n, i);
+        auto tokens = [&](auto whole) {
 #pragma unroll
-        for (int j = PIECE - 1; j >= 0; j--) {
-            ss[j] = 0.0f;
+            for (int j = PIECE - 1; j >= 0; j--) {
+                ss[j] = 0.0f;
+                if (!decltype(whole)::value && tp + j >= t1) continue;
 #pragma unroll
-            for (int i = 0; i < V; i++) {
-                float acc = 0.0f;
+                for (int i = 0; i < V; i++) {
+                    float acc = 0.0f;
 #pragma unroll
-                for (int n = TAPS - 1; n >= 0; n--) acc = fmaf(input(j - n, i), w[n][i], acc);
-                in[j][i] = mine ? __fdividef(acc, 1.0f + expf(-acc)) : 0.0f;
-                ss[j] = fmaf(in[j][i], in[j][i], ss[j]);
+                    for (int n = TAPS - 1; n >= 0; n--) acc = fmaf(input(j - n, i), w[n][i], acc);
+                    in[j][i] = mine ? __fdividef(acc, 1.0f + expf(-acc)) : 0.0f;
+                    ss[j] = fmaf(in[j][i], in[j][i], ss[j]);
+                }
             }
-        }
+        };
+        // tokens that are not there cost as much as those that are: two tokens of 4096 channels 6.0 us computed as eight, 3.6 as two, 3 x 5 6.1 and 5.6 as five
+        if (PIECE < 8 || tp + PIECE <= t1) tokens(std::true_type());
+        else tokens(std::false_type());
 #pragma unroll
         for (int n = 1; n < TAPS; n++)
 #pragma unroll
@@ -194,9 +228,11 @@ __global__ void __launch_bounds__(128, conv_ctas(V, TAPS, PIECE, SRC)) ns_short_
             if constexpr (PIECE == 8) f = g.scale / sqrtf(conv_sum8(ss, lane) + 1e-6f);
             else f = g.scale / sqrtf(ns_warp_sum(ss[0]) + 1e-6f);
         }
+        float f1 = 1.0f;
+        if (PIECE == 2 && g.unit) f1 = g.scale / sqrtf(ns_warp_sum(ss[PIECE - 1]) + 1e-6f);
 #pragma unroll
         for (int j = 0; j < PIECE; j++) {
-            const float fj = PIECE == 8 ? __shfl_sync(0xffffffffu, f, j * 4) : f;
+            const float fj = PIECE == 8 ? __shfl_sync(0xffffffffu, f, j * 4) : (j == 1 ? f1 : f);
             if (!mine || tp + j >= t1) continue;
             T* out = reinterpret_cast<T*>(g.out) + ((int64_t)b * a.steps + tp + j) * g.out_ld + ch;
             if constexpr (V == 4) {
@@ -640,6 +676,7 @@ extern "C" int ns_short_conv(ns_device_t h, uint64_t src, int splits, int src_dt
                         return v == 1 ? slide(ns_short_conv_slide_kernel<T, 1, 4, P, S>) : (v == 2 ? slide(ns_short_conv_slide_kernel<T, 2, 4, P, S>) : slide(ns_short_conv_slide_kernel<T, 4, 4, P, S>));
                     return v == 1 ? slide(ns_short_conv_slide_kernel<T, 1, 8, P, S>) : (v == 2 ? slide(ns_short_conv_slide_kernel<T, 2, 8, P, S>) : slide(ns_short_conv_slide_kernel<T, 4, 8, P, S>));
                 };
+                if (steps == 2) return of(std::integral_constant<int, 2>());
                 return steps == 1 ? of(std::integral_constant<int, 1>()) : of(std::integral_constant<int, CONV_WARP>());
             };
             return together ? any(std::integral_constant<int, CONV_SLABS>()) : any(std::integral_constant<int, CONV_ANY>());

@@ -183,6 +183,38 @@ def test_short_convolution_of_one_bf16_matrix(dev, steps, taps, hd, ragged):
             assert np.array_equal(after[i, t % taps], x[i, t])
 
 
+@pytest.mark.parametrize("steps", [1, 2, 3, 7, 8, 9, 35])
+@pytest.mark.parametrize("taps,hd", [(2, 24), (4, 32), (7, 32), (3, 48), (4, 64), (6, 64), (4, 96), (8, 128)])
+@pytest.mark.parametrize("dtype,splits", [("bf16", 1), ("f32", 1), ("f32", 2), ("f32", 4)])
+def test_short_convolution_of_few_tokens(dev, steps, taps, hd, dtype, splits):
+    """A step of one or two tokens has builds of its own, a piece of three to seven is computed token by token, and heads of up to 64 channels widen bf16 inputs
+    together; with an earlier token in the history."""
+    B, heads, before = 2, 5, 3
+    c = heads * hd
+    rng = rng_for(8, steps, taps, hd)
+    parts = rng.standard_normal((splits, B, steps, c)).astype(np.float32)
+    if dtype == "bf16":
+        parts = f32(bf16_bits(parts))
+    x = np.concatenate([rng.standard_normal((B, before, c)).astype(np.float32), sum(parts[1:], parts[0])], 1)
+    w = rng.standard_normal((c, taps)).astype(np.float32)
+    src = dev.from_numpy(bf16_bits(parts) if dtype == "bf16" else parts)
+    hist = np.zeros((B, taps, c), np.float32)
+    for t in range(before):
+        hist[:, t % taps] = x[:, t]
+    dh, out, dw = dev.from_numpy(hist), dev.empty(B * steps * c), dev.from_numpy(w)
+    slots, pos = dev.from_numpy(np.arange(B, dtype=np.int32)), dev.from_numpy(np.full(B, before, np.int32))
+    fields = (C.c_int64 * 9)(0, heads, hd, taps, 1, dw.ptr, dh.ptr, out.ptr, c)
+    N.call("ns_short_conv", dev.handle, u(src.ptr), splits, N.NS_BF16 if dtype == "bf16" else N.NS_F32, c, 1, fields, (C.c_float * 1)(0.5), i64(taps * c), u(slots.ptr),
+           u(pos.ptr), B, steps, N.NS_F32)
+    dev.synchronize()
+    got, after = out.download((B, steps, c)), dh.download((B, taps, c))
+    for i in range(B):
+        want = F.unit(F.short_conv(x[i].astype(np.float64), w.astype(np.float64)).reshape(-1, heads, hd)).reshape(-1, c)[before:] * 0.5
+        close(got[i], want, 1e-5)
+        for t in range(max(0, before + steps - taps + 1), before + steps):
+            assert np.array_equal(after[i, t % taps], x[i, t])
+
+
 # ------------------------------------------------------------------------------------------------ delta rule
 def run_delta(dev, data, cuts, H, kv, dim, vdim, channelwise, slots=(0,), chunk_from=1 << 30):
     """o [B, T, H, vdim] and final states, the sequences fed in `cuts`."""

@@ -392,10 +392,12 @@ int launch_decode(NsDevice* d, const DecodeParams& p)
     };
     // Builds: four CTAs an SM, or five (the query reloaded for each chunk, 96 registers) where that leaves fewer or smaller last waves; four rounds of loads in flight
     // where a CTA's own chain of loads is what its time consists of (measured: 384 CTAs gain 9 %, 512 lose 30 % with four rounds).  Five against
-    // four an SM, us: 2048 CTAs x 4096 positions 603, 655; 640 x 300 20.6, 28; 1024 x 576 58, 53; 1536 x 700 99, 92.
+    // four an SM, us: 2048 CTAs x 4096 positions 603, 655; 640 x 300 20.6, 28; 1024 x 576 58, 53; 1536 x 700 99, 92.  Heads of 32 columns leave a CTA little to
+    // wait for, and past three waves of four the fifth counts for more than the last wave: 8192 x 100 77.7, 87.8; 2880 x 128 27.9, 30.6; 2400 x 700 68.6,
+    // 75.1; 1760 x 40 18.1, 17.3; 1024 x 576 28.9, 28.0.
     int rc;
     if (ctas < 3 * (int64_t)d->sm_count) rc = launch(ns_attention_decode_kernel<DH, 4, 3>);
-    else if (cost(5) < cost(4)) rc = launch(ns_attention_decode_kernel<DH, 2, 5>);
+    else if (cost(5) < cost(4) || (DH == 32 && ctas > 12 * (int64_t)d->sm_count)) rc = launch(ns_attention_decode_kernel<DH, 2, 5>);
     else rc = launch(ns_attention_decode_kernel<DH, 2, 4>);
     if (rc != NS_OK) return rc;
     if (p.splits > 1) {

@@ -200,7 +200,7 @@ def test_a_sequence_in_a_batch_equals_the_sequence_in_a_small_batch(dev, orc, ca
 
 
 @pytest.mark.parametrize("dh", [32, 64, 128])
-@pytest.mark.parametrize("B", [28, 40, 64])      # 448, 640 and 1024 rows of 16 heads: four CTAs an SM, five, four
+@pytest.mark.parametrize("B", [28, 40, 64, 120]) # 448, 640, 1024 and 1920 rows of 16 heads: four CTAs an SM, five, four, four or (heads of 32 columns) five
 @pytest.mark.parametrize("cap,length", [(128, 1), (128, 65), (640, 333)])
 def test_builds_for_many_rows(dev, orc, dh, B, cap, length):
     """The builds for many rows against the split rows of few, bit for bit, and the oracle: one position, a chunk's last few, two chunks."""

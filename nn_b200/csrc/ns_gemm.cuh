@@ -62,7 +62,7 @@ int ns_stream_i8_run(NsDevice* d, const NsGemmParams& p, const void* a, const vo
 
 // The streaming bf16 kernel (ns_stream_bf16.cu): weights [N, K], one launch, K summed inside the CTA.  `p` must hold M, N, K, the epilogue
 // fields and out (float or bf16).
-bool ns_stream_bf16_fits(const NsDevice* d, int M, int N, int K);
+bool ns_stream_bf16_fits(const NsDevice* d, int M, int N, int K, bool deferred);
 int ns_stream_bf16_run(NsDevice* d, const NsGemmParams& p, const void* a, const void* w);
 
 #ifdef __CUDACC__

@@ -1093,7 +1093,7 @@ int ns_gemm_run(NsDevice* d, int kind, const void* a, const void* b, bool b_is_k
         ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0)
         return ns_stream_i8_run(d, p, a, b);
     // Few rows of bf16 against [N, K] weights: the streaming kernel, one slab when the epilogue is deferred.
-    if (kind == NS_KIND_BF16 && !b_is_kn && d->force_bn == 0 && d->force_splits == 0 && ns_stream_bf16_fits(d, M, N, K) &&
+    if (kind == NS_KIND_BF16 && !b_is_kn && d->force_bn == 0 && d->force_splits == 0 && ns_stream_bf16_fits(d, M, N, K, deferred) &&
         ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0) {
         if (deferred) {
             void* slab = nullptr;

@@ -28,7 +28,7 @@ constexpr int SB_THREADS = SB_WARPS * 32;
 constexpr int SB_TILE = 16;          // output columns per tile
 constexpr int SB_UNIT = 128;         // elements of K per unit
 constexpr int SB_PITCH = 20;         // floats per activation row of a slot (16 columns): 8 q + g meets every bank once
-constexpr size_t SB_SMEM_MAX = 227 * 1024;
+constexpr size_t SB_SMEM_MAX = 164 * 1024;    // see ns_stream_bf16_fits
 
 __host__ __device__ constexpr int sb_slot_floats(int groups) { return groups * 8 * SB_PITCH; }
 
@@ -205,17 +205,28 @@ int launch_stream_bf16(NsDevice* d, const NsGemmParams& p, const void* a, const 
 
 }  // namespace
 
-// Up to eight rows: every size whose activations and slots fit shared memory.  Nine to sixteen: short rows and few columns only.  There
-// the tcgen05 kernel is as fast or faster elsewhere, because a CTA of this one copies all the activations (16 x 5632: 180 KB) and adds
-// the sums of all its tiles before anything is stored.  Measured with the row kernel that follows, us, tcgen05 against this:
+// Up to eight rows: every size whose activations and slots leave L1 a quarter of an SM's 256 KB, because the weights in flight (128 KB
+// a SM at most) pass through it.  us, tcgen05 against this, 1 and 8 rows:
+//   2048 x 8192 11.5, 7.5 and 11.6, 8.7;  4096 x 9216 17.9, 14.4 and 18.1, 15.6;  4096 x 11264 20.1, 19.7 and 20.5, 21.2;  4096 x 12288 21.6, 37.1 and 22.1, 38.8
+// Not where tiles divide badly and K is long: the bytes of weights that the busiest CTA has beyond an even share are time in which the others
+// wait.  In front of a row kernel, which reads split sums almost as fast as whole ones, the tcgen05 kernel is ahead sooner.  (With the row kernel) 8 rows:
+//   4096 x 4096 (34 KB) 13.6, 12.4;  768 x 8192 (172 KB) 9.1, 9.4;  1024 x 8192 (145 KB) 9.2, 9.8;  2400 x 4096 (126 KB) 10.7, 11.0;  2400 x 5120 (157 KB) 11.3, 12.0
+//   2400 x 8192 (252 KB) 13.6, 16.2, and alone 12.2, 13.3;  3000 x 8192 (186 KB) alone 13.4, 13.0;  1 row: 768 x 8192 9.1, 8.3;  2400 x 8192 13.5, 14.6
+// Nine to sixteen rows: short rows and few columns only.  There the tcgen05 kernel is as fast or faster elsewhere, because a CTA of this one copies
+// all the activations (16 x 5632: 180 KB) and adds the sums of all its tiles before anything is stored.  With the row kernel that follows, us:
 //   8 rows:  2048 x 2048 7.1, 6.4;  11264 x 2048 16.8, 15.2;  2048 x 5632 9.3, 9.4;  32000 x 5632 65.5, 61.0 (floor 55.8);  1 row: 64.4, 58.1
-//   16 rows: 2048 x 2048 7.1, 6.9;  3088 x 1024 7.1, 6.4;  6176 x 2048 11.9, 12.3;  32000 x 2048 28.1, 29.7;  2048 x 5632 9.3, 14.3
-// In a chain of products alone (8 rows): 12.4, 9.4;  7.1, 3.8;  9.5, 6.3 us (11264 x 2048, 2048 x 2048, 2048 x 5632); 14336 x 4096 23.5, 20.8.
-bool ns_stream_bf16_fits(const NsDevice* d, int M, int N, int K)
+//   16 rows: 2048 x 2048 7.7, 7.0;  3088 x 1024 8.6, 7.6;  3088 x 2048 10.1, 9.3;  4096 x 2048 10.4, 10.1;  6176 x 2048 11.9, 12.3;  32000 x 2048 28.1, 29.7
+//            2048 x 5632 9.3, 14.3;  2400 x 2048 (63 KB) 8.6, 8.8;  2600 x 2048 (57 KB) 9.0, 8.7
+// In a chain of products alone (8 rows): 12.4, 9.4;  7.1, 3.8;  9.5, 6.3 us (11264 x 2048, 2048 x 2048, 2048 x 5632); 14336 x 4096 23.5, 20.8; 16 rows
+// of 4096 x 2048 8.3, 5.7, of 3088 x 1024 6.8, 4.1.
+bool ns_stream_bf16_fits(const NsDevice* d, int M, int N, int K, bool deferred)
 {
     if (M < 1 || M > 16 || K % 8 != 0) return false;
     if (M > 8 && (K > 2048 || N > 4096)) return false;
-    return sb_smem_bytes(d->sm_count, M <= 8 ? 1 : 2, N, K) <= SB_SMEM_MAX;
+    if (sb_smem_bytes(d->sm_count, M <= 8 ? 1 : 2, N, K) > SB_SMEM_MAX) return false;
+    const int64_t tiles = (N + SB_TILE - 1) / SB_TILE, most = (tiles + d->sm_count - 1) / d->sm_count;
+    const int64_t beyond = (most * d->sm_count - tiles) * K * (SB_TILE * 2) / d->sm_count;     // bytes
+    return beyond <= (!deferred ? 230 : M <= 4 ? 220 : M <= 8 ? 120 : 62) * 1024;
 }
 
 int ns_stream_bf16_run(NsDevice* d, const NsGemmParams& p, const void* a, const void* w)

@@ -21,7 +21,7 @@ def _wide(b):
 
 
 @pytest.mark.parametrize("n,k", [(8, 8), (16, 128), (24, 72), (40, 1032), (1000, 264), (2368, 2048), (2376, 136), (4096, 2048), (4104, 2048), (2048, 5632),
-                                 (4800, 5120), (32000, 256)])
+                                 (4800, 5120), (32000, 256), (768, 8192), (2400, 8192), (2048, 9216), (2048, 10240)])
 def test_products(dev, n, k):
     rng = np.random.default_rng(n * 7 + k)
     w = _bf16(rng.standard_normal((n, k)))
@@ -46,8 +46,10 @@ def test_products(dev, n, k):
         N.call("ns_d2d_async", dev.handle, u64(slabs.ptr), ptr, u64(4 * splits.value * m * n))
         dev.synchronize()
         slabs = slabs.download((splits.value, m, n))
-        if m <= 8:
+        # tiles that divide badly and rows that are too long are split for the row kernel, and from some length on for a finished matrix too
+        if m <= 8 and (n, k) not in ((4800, 5120), (768, 8192), (2400, 8192), (2048, 10240)):
             assert splits.value == 1 and np.array_equal(slabs[0], y[:m])
+        assert np.all(np.abs(slabs.astype(np.float64).sum(0) - a @ wide.T) <= (k + 16) * 2.0 ** -22 * (np.abs(a) @ np.abs(wide).T))
         rows[m] = y[0]
         d_b = dev.empty(m * n, N.NS_BF16)
         N.call("ns_linear_forward", dev.handle, h, u64(d_x.ptr), u64(0), m, N.EPI_NONE, u64(0), N.NS_F32, N.NS_BF16, u64(d_b.ptr))

@@ -61,9 +61,10 @@ __global__ void __launch_bounds__(128) ns_embed_ngram_kernel(const int32_t* __re
     }
 }
 
-// The RMS row kernels of few rows are launched while the product in front of them still runs: generating with 7 sequences (topidra), 64 tokens,
-// 15.5 -> 15.0 ms (seven rows of 2048 with both norms, in a chain of their own, 3.2 -> 2.3 us); with 64 (fabezen) level, so from nine rows
-// on they wait, as the products in front then are other kernels.
+// The RMS row kernels of few rows are launched while the product in front of them still runs, where that left one slab (ns_stream_bf16.cu):
+// generating with 7 sequences (topidra), 64 tokens, 15.5 -> 15.0 ms (seven rows of 2048 with both norms, in a chain of their own, 3.2 -> 2.3 us).  Behind a
+// product that split K all rows can land on the one SM that it left free: 8 x 2600 x 5120 with its row kernel 12.7 us so, 11.3 waiting; and with 64
+// rows (fabezen) it is level.
 constexpr unsigned RMS_EARLY_ROWS = 8;
 // Their vectors towards L2, before the wait: a hint, nothing is read.
 NS_DEVINL void rms_prefetch(const float* v, const float* w, int cols)
@@ -88,6 +89,7 @@ struct RmsArgs {
     int cols;
     void* y;
     int64_t y_ld;
+    bool early;              // launched beside the product in front
 };
 
 template <typename T, bool VEC, int SLABS>
@@ -99,6 +101,7 @@ __global__ void __launch_bounds__(256) ns_rms_rows_kernel(const RmsArgs a)
     // asked for now, read after the reduction (see ns_rms_post_rows_vec_kernel)
     if (VEC && SLABS != NS_ONE_SLAB) rms_prefetch(nullptr, a.w, a.cols);
     ns_pdl_wait();
+    if (!a.early) ns_pdl_trigger();
     const float* norm_w = SLABS != NS_ONE_SLAB ? ns_after_wait(a.w) : a.w;
     const int row = a.row_map != nullptr ? a.row_map[blockIdx.x] : (int)blockIdx.x;
     const int64_t base = (int64_t)row * a.cols;
@@ -123,7 +126,7 @@ __global__ void __launch_bounds__(256) ns_rms_rows_kernel(const RmsArgs a)
             buf[c] = v;
         }
     }
-    ns_pdl_trigger();       // not before the row is here (see ns_rms_post_rows_vec_kernel)
+    if (a.early) ns_pdl_trigger();       // (see ns_rms_post_rows_vec_kernel)
     if (a.w == nullptr) return;
     ss = ns_cta_sum(ss, red);
     const float inv = 1.0f / sqrtf(ss / (float)a.cols + a.eps);
@@ -159,6 +162,7 @@ __global__ void __launch_bounds__(256) ns_rms_post_rows_vec_kernel(const PostRms
     // (the build for one slab is never launched early, and left to schedule these loads as it likes)
     if (SLABS != NS_ONE_SLAB) rms_prefetch(p.post_w, a.w, a.cols);
     ns_pdl_wait();
+    if (!a.early) ns_pdl_trigger();
     const float *post_w = SLABS != NS_ONE_SLAB ? ns_after_wait(p.post_w) : p.post_w, *norm_w = SLABS != NS_ONE_SLAB ? ns_after_wait(a.w) : a.w;
     const int row = blockIdx.x;
     const int64_t base = (int64_t)row * a.cols;
@@ -191,8 +195,10 @@ __global__ void __launch_bounds__(256) ns_rms_post_rows_vec_kernel(const PostRms
     for (int i = 0; i < Q; i++) { ss = fmaf(s[i].x, s[i].x, ss); ss = fmaf(s[i].y, s[i].y, ss); ss = fmaf(s[i].z, s[i].z, ss); ss = fmaf(s[i].w, s[i].w, ss); }
     const float post = 1.0f / sqrtf(ns_cta_sum(ss, red[0]) / (float)a.cols + a.eps);
     // The product that follows starts at this signal and asks for its first weights, up to 19 MB.  Given before this row has arrived, the
-    // row's loads (the norms' weights come from HBM) queue behind them: 5.1 us against 3.6 for seven rows of 2048.
-    ns_pdl_trigger();
+    // row's loads (the norms' weights come from HBM) queue behind them: 5.1 us against 3.6 for seven rows of 2048.  But where this kernel waited for the
+    // product in front, the next one's start is worth more: 9 to 64 rows of a 2048 x 5632 product and this 11.1 to 11.5 us with the signal here, 9.8 to 10.1
+    // with it at the start, as without a row kernel; fabezen with 64 sequences 25.9 and 25.5 ms.
+    if (a.early) ns_pdl_trigger();
     ss = 0.0f;
 #pragma unroll
     for (int i = 0; i < Q; i++) {
@@ -415,11 +421,12 @@ extern "C" int ns_rms_rows(ns_device_t h, uint64_t x, uint64_t src, int splits, 
     a.cols = cols;
     a.y = reinterpret_cast<void*>(y);
     a.y_ld = y_ld;
+    a.early = rows <= RMS_EARLY_ROWS && a.src.splits == 1;
     const bool vec = ((cols | (src ? src_ld : 0) | (w ? y_ld : 0)) & 3) == 0 && ((x | src | x_out | w | y) & 15) == 0 && (a.src.slab & 3) == 0;
     const size_t smem = (size_t)((cols + 3) & ~3) * 4;
     auto launch = [&](auto kernel) -> int {
         if (smem > 48 * 1024) NS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (rows <= RMS_EARLY_ROWS) NS_CUDA(ns_launch_pdl(kernel, dim3((unsigned)rows), dim3(256), smem, d->stream, a));
+        if (a.early) NS_CUDA(ns_launch_pdl(kernel, dim3((unsigned)rows), dim3(256), smem, d->stream, a));
         else NS_CUDA(ns_launch_plain(kernel, dim3((unsigned)rows), dim3(256), smem, d->stream, a));
         return NS_OK;
     };
@@ -451,13 +458,14 @@ extern "C" int ns_rms_post_rows(ns_device_t h, uint64_t x, uint64_t src, int spl
     a.cols = cols;
     a.y = reinterpret_cast<void*>(y);
     a.y_ld = y_ld;
+    a.early = rows <= RMS_EARLY_ROWS && a.src.splits == 1;
     p.post_w = reinterpret_cast<const float*>(post_w);
     p.plus = reinterpret_cast<const float*>(plus);
     const bool vec = ((cols | src_ld | (w ? y_ld : 0)) & 3) == 0 && ((x | src | x_out | w | y | post_w | plus) & 15) == 0 && (a.src.slab & 3) == 0 && cols <= 8192;
     const size_t smem = vec ? 0 : (size_t)((cols + 3) & ~3) * 4;
     auto launch = [&](auto kernel) -> int {
         if (smem > 48 * 1024) NS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (rows <= RMS_EARLY_ROWS) NS_CUDA(ns_launch_pdl(kernel, dim3((unsigned)rows), dim3(256), smem, d->stream, p));
+        if (a.early) NS_CUDA(ns_launch_pdl(kernel, dim3((unsigned)rows), dim3(256), smem, d->stream, p));
         else NS_CUDA(ns_launch_plain(kernel, dim3((unsigned)rows), dim3(256), smem, d->stream, p));
         return NS_OK;
     };

@@ -66,6 +66,9 @@ __global__ void __launch_bounds__(128) ns_embed_ngram_kernel(const int32_t* __re
 // product that split K all rows can land on the one SM that it left free: 8 x 2600 x 5120 with its row kernel 12.7 us so, 11.3 waiting; and with 64
 // rows (fabezen) it is level.
 constexpr unsigned RMS_EARLY_ROWS = 8;
+// Not rows that are long in coming: the product behind waits for the late signal (see ns_rms_post_rows_vec_kernel), and 8 x 12000 x 2048 with its row kernel
+// took 21.3 us for 20.4, 8 x 9000 x 2048 16.3 for 15.5 (8 x 8192 x 2048 15.5 both ways).
+static bool rms_early(int64_t rows, int cols, int splits) { return rows <= RMS_EARLY_ROWS && splits == 1 && cols <= 8192; }
 // Their vectors towards L2, before the wait: a hint, nothing is read.
 NS_DEVINL void rms_prefetch(const float* v, const float* w, int cols)
 {
@@ -421,7 +424,7 @@ extern "C" int ns_rms_rows(ns_device_t h, uint64_t x, uint64_t src, int splits, 
     a.cols = cols;
     a.y = reinterpret_cast<void*>(y);
     a.y_ld = y_ld;
-    a.early = rows <= RMS_EARLY_ROWS && a.src.splits == 1;
+    a.early = rms_early(rows, cols, a.src.splits);
     const bool vec = ((cols | (src ? src_ld : 0) | (w ? y_ld : 0)) & 3) == 0 && ((x | src | x_out | w | y) & 15) == 0 && (a.src.slab & 3) == 0;
     const size_t smem = (size_t)((cols + 3) & ~3) * 4;
     auto launch = [&](auto kernel) -> int {
@@ -458,7 +461,7 @@ extern "C" int ns_rms_post_rows(ns_device_t h, uint64_t x, uint64_t src, int spl
     a.cols = cols;
     a.y = reinterpret_cast<void*>(y);
     a.y_ld = y_ld;
-    a.early = rows <= RMS_EARLY_ROWS && a.src.splits == 1;
+    a.early = rms_early(rows, cols, a.src.splits);
     p.post_w = reinterpret_cast<const float*>(post_w);
     p.plus = reinterpret_cast<const float*>(plus);
     const bool vec = ((cols | src_ld | (w ? y_ld : 0)) & 3) == 0 && ((x | src | x_out | w | y | post_w | plus) & 15) == 0 && (a.src.slab & 3) == 0 && cols <= 8192;

@@ -9,6 +9,8 @@
 // The reference runs each of these with one thread per row; here a CTA handles a row.
 #include <math.h>
 
+#include <atomic>
+
 #include "ns_common.cuh"
 #include "ns_rows.cuh"
 
@@ -186,23 +188,37 @@ __global__ void ns_layernorm_q_reg_kernel(const uint16_t* __restrict__ x, const 
 
 inline unsigned grid_rows(const NsDevice* d, int64_t rows);
 
+// Many float rows, two vectors a thread: the next row is in registers while this one is reduced, and as many CTAs as are resident walk the rows.  For every
+// width that two vectors a thread and whole warps make up, up to 1024 threads: 2560, 3072, ... 16384.  Those without a register kernel of their own
+// (row_shape) gain most, from eight rows an SM on: 8192 x 2560 35.2 -> 17.4 us, 8192 x 5120 61 -> 34.3, 3000 x 7168 31.5 -> 20.8, 1184 x 3072 7.0 -> 5.2.
+// 4096 columns have one, whose CTAs are more and free sooner: they change over where the rows no longer come out of L2 (8192 rows 32.5 -> 27.7 us, 5000 19.7 -> 17.4, 4000
+// 14.6 -> 14.2, 3000 11.1 and 11.2, 2000 8.2 and 9.0).  2048 and 8192 stay: one vector leaves room for more CTAs (8192 x 2048: 17.9, 19.7
+// so), four need few (2000 x 8192 13.4, 16.2 with 512 threads of two; 8192 rows 57.8, 56.1).
+bool quantize_ahead_fits(const NsDevice* d, int64_t rows, int cols)
+{
+    if (cols % 512 != 0 || cols <= 2048 || cols > 16384) return false;
+    unsigned threads;
+    int vpt;
+    return rows >= (ns_rows::row_shape(cols, &threads, &vpt) ? (vpt == 2 ? 27 : INT32_MAX) : 8) * (int64_t)d->sm_count;
+}
+cudaError_t launch_quantize_ahead(NsDevice* d, const float* x, int64_t rows, int cols, int8_t* q, float* scale)
+{
+    // CTAs an SM holds, by device and warps of a CTA (any thread may find them, all find the same)
+    static std::atomic<int> held[64][33];
+    std::atomic<int>& known = held[d->ordinal][cols / 512];
+    int ctas = known.load(std::memory_order_relaxed);
+    if (ctas == 0) {
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, ns_quantize_rows_reg_kernel<2, true, true>, cols / 16, 0);
+        if (e != cudaSuccess) return e;
+        known.store(ctas, std::memory_order_relaxed);
+    }
+    return ns_launch_plain(ns_quantize_rows_reg_kernel<2, true, true>, dim3((unsigned)(d->sm_count * ctas)), dim3(cols / 16), 0, d->stream, x, rows, cols, q, scale);
+}
+
 template <bool F32IN>
 cudaError_t launch_quantize_reg(NsDevice* d, unsigned threads, int vpt, const void* x, int64_t rows, int cols, int8_t* q, float* scale)
 {
     const dim3 grid(grid_rows(d, rows)), block(threads);
-    // Many float rows of two vectors a thread: the next row is in registers while this one is reduced, and as many CTAs as are resident walk the rows
-    // (8192 x 4096: 32.1 -> 27.5 us, 6.1 TB/s; 3000 rows 12.8 -> 12.3).  With one vector more CTAs fit and are ahead without it (8192 x 2048: 17.9, 19.7
-    // with it), with four the registers are missing (4000 x 8192: 30.0, 32.3).
-    if (F32IN && vpt == 2 && rows >= 8 * (int64_t)d->sm_count) {
-        static int ctas = 0;             // an SM holds
-        if (ctas == 0) {
-            int n = 0;
-            const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ns_quantize_rows_reg_kernel<2, F32IN, true>, 256, 0);
-            if (e != cudaSuccess) return e;
-            ctas = n < 1 ? 1 : n;
-        }
-        return ns_launch_plain(ns_quantize_rows_reg_kernel<2, F32IN, true>, dim3((unsigned)(d->sm_count * ctas)), block, 0, d->stream, x, rows, cols, q, scale);
-    }
     switch (vpt) {
         case 1: return ns_launch_plain(ns_quantize_rows_reg_kernel<1, F32IN, false>, grid, block, 0, d->stream, x, rows, cols, q, scale);
         case 2: return ns_launch_plain(ns_quantize_rows_reg_kernel<2, F32IN, false>, grid, block, 0, d->stream, x, rows, cols, q, scale);
@@ -416,6 +432,10 @@ extern "C" int ns_quantize_rows_i8(ns_device_t h, uint64_t x, int in_dtype, int6
     int vpt = 0;
     if (in_dtype == NS_BF16 && ((x | q) & 15) == 0 && ns_rows_stream_fits(false, rows, cols)) {
         NS_CUDA(ns_rows_stream_quantize(d, reinterpret_cast<const uint16_t*>(x), rows, cols, reinterpret_cast<int8_t*>(q), reinterpret_cast<float*>(scale)));
+        return NS_OK;
+    }
+    if (in_dtype == NS_F32 && ((x | q) & 15) == 0 && quantize_ahead_fits(d, rows, cols)) {
+        NS_CUDA(launch_quantize_ahead(d, reinterpret_cast<const float*>(x), rows, cols, reinterpret_cast<int8_t*>(q), reinterpret_cast<float*>(scale)));
         return NS_OK;
     }
     if (((x | q) & 15) == 0 && ns_rows::row_shape(cols, &threads, &vpt)) {

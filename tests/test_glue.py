@@ -199,13 +199,13 @@ def test_embed_pos_of_bf16_tables(dev, orc, batch, steps, dim):
     assert np.array_equal(y.download((batch, steps, dim)), exp)
 
 
-@pytest.mark.parametrize("rows", [1183, 1184, 1185, 2400])
-def test_quantize_many_float_rows_a_row_ahead(dev, orc, rows):
-    """Eight rows an SM and more: the CTAs walk the rows with the next one in registers.  The same bytes and scales as for few rows at a time,
-    rows with a NaN, an infinity, zeros or subnormal values among them."""
-    cols = 4096
+@pytest.mark.parametrize("rows,cols", [(1183, 2560), (1184, 2560), (1185, 3072), (2400, 3584), (1500, 5120), (1300, 7168), (1184, 16384), (2400, 4096), (3995, 4096),
+                                       (3996, 4096), (4001, 4096), (1300, 8192), (1300, 2816)])
+def test_quantize_many_float_rows_a_row_ahead(dev, orc, rows, cols):
+    """Eight rows an SM and more (4096 columns: 27): the CTAs walk the rows with the next one in registers.  The same bytes and scales as for few rows at a
+    time, rows with a NaN, an infinity, zeros or subnormal values among them."""
     x = orc.normal((rows, cols), 84, 1.5)
-    x[5, 7], x[6, 4095], x[7], x[8] = np.nan, np.inf, 0.0, 1e-41
+    x[5, 7], x[6, cols - 1], x[7], x[8] = np.nan, np.inf, 0.0, 1e-41
     dx, dq, ds, dq2, ds2 = dev.from_numpy(x), dev.empty(rows * cols, N.NS_I8), dev.empty(rows), dev.empty(rows * cols, N.NS_I8), dev.empty(rows)
     N.call("ns_quantize_rows_i8", dev.handle, dx.ptr, N.NS_F32, C.c_int64(rows), cols, dq.ptr, ds.ptr)
     for r0 in range(0, rows, 600):

@@ -101,6 +101,7 @@ ns_stream_bf16_kernel(const NsGemmParams p, const uint16_t* __restrict__ a, cons
     ns_pdl_wait();
     ns_pdl_trigger();
     a = ns_after_wait(a);
+    const float* bias = ns_after_wait(p.bias);              // a product's bias may be the previous kernel's, too
     if (!p.prefetch_b) fill();
 
     // activations to shared memory, zeros behind K
@@ -172,7 +173,7 @@ ns_stream_bf16_kernel(const NsGemmParams p, const uint16_t* __restrict__ a, cons
         }
         const int n = tile_begin * SB_TILE + c;
         const size_t at = (size_t)m * p.N + n;
-        if (p.epilogue != NS_EPI_NONE) v = __fadd_rn(v, __ldg(&p.bias[n]));
+        if (p.epilogue != NS_EPI_NONE) v = __fadd_rn(v, __ldg(&bias[n]));
         if (p.epilogue == NS_EPI_BIAS_GELU) v = ns_gelu_fast(v);
         if (p.epilogue == NS_EPI_BIAS_RESIDUAL) v = __fadd_rn(v, ns_gemm_residual(p, at));
         if (p.out_dtype == NS_F32) reinterpret_cast<float*>(p.out)[at] = v;

@@ -213,7 +213,11 @@ int launch_stream_bf16(NsDevice* d, const NsGemmParams& p, const void* a, const 
 // wait.  In front of a row kernel, which reads split sums almost as fast as whole ones, the tcgen05 kernel is ahead sooner.  (With the row kernel) 8 rows:
 //   4096 x 4096 (34 KB) 13.6, 12.4;  768 x 8192 (172 KB) 9.1, 9.4;  1024 x 8192 (145 KB) 9.2, 9.8;  2400 x 4096 (126 KB) 10.7, 11.0;  2400 x 5120 (157 KB) 11.3, 12.0
 //   2400 x 8192 (252 KB) 13.6, 16.2, and alone 12.2, 13.3;  3000 x 8192 (186 KB) alone 13.4, 13.0
-// (One row would gain up to 220 KB, 768 x 8192 9.1, 8.3; but one line for one to eight rows keeps a row's bits the same among them.)
+// (One row would gain up to 220 KB, 768 x 8192 9.1, 8.3, and with many columns, 64000 x 1024 24.9, 23.0; but one line for one to eight rows keeps a row's
+// bits the same among them.)
+// Not many columns over rows of 512 to 1024, where a CTA's 2 400 outputs and more, which it adds up after its last weights, are not made up for: 8 rows
+// 100000 x 512 20.8, 23.6;  128256 x 1024 45.1, 48.9;  64000 x 1024 25.7, 26.6;  32000 x 1024 14.2, 14.0.  Shorter rows are tiles of one or two steps to the
+// tcgen05 kernel (200000 x 128 25.1, 18.2;  50000 x 256 11.3, 8.8), longer ones weigh more than the outputs (64000 x 2048 47.6, 46.5;  128256 x 4096 174, 167).
 // Nine to sixteen rows: short rows and few columns only.  There the tcgen05 kernel is as fast or faster elsewhere, because a CTA of this one copies
 // all the activations (16 x 5632: 180 KB) and adds the sums of all its tiles before anything is stored.  With the row kernel that follows, us:
 //   8 rows:  2048 x 2048 7.1, 6.4;  11264 x 2048 16.8, 15.2;  2048 x 5632 9.3, 9.4;  32000 x 5632 65.5, 61.0 (floor 55.8);  1 row: 64.4, 58.1
@@ -227,6 +231,7 @@ bool ns_stream_bf16_fits(const NsDevice* d, int M, int N, int K, bool deferred)
     if (M > 8 && (K > 2048 || N > 4096)) return false;
     if (sb_smem_bytes(d->sm_count, M <= 8 ? 1 : 2, N, K) > SB_SMEM_MAX) return false;
     const int64_t tiles = (N + SB_TILE - 1) / SB_TILE, most = (tiles + d->sm_count - 1) / d->sm_count;
+    if (M <= 8 && K > 256 && K < 2048 && most * SB_TILE * 8 > 2400) return false;
     const int64_t beyond = (most * d->sm_count - tiles) * K * (SB_TILE * 2) / d->sm_count;     // bytes
     return beyond <= (!deferred ? 230 : M <= 8 ? 120 : 62) * 1024;
 }
